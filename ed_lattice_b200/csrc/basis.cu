@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
+#include <map>
 #include <mutex>
 #include <tuple>
 
@@ -356,7 +357,7 @@ int build_spin(edg_sector_s* s, int spin, SpinBasis& B, int nel) {
   return EDG_OK;
 }
 
-int build_sell(edg_sector_s* s, SpinBasis& B);
+int build_sell(edg_sector_s* s, SpinBasis& B, bool up);
 
 int build_tables(edg_sector_s* s, int spin, SpinBasis& B) {
   cudaStream_t st = s->stream;
@@ -401,8 +402,7 @@ int build_tables(edg_sector_s* s, int spin, SpinBasis& B) {
                                      B.off.p, B.src.p, B.val64.p, B.val32.p, B.val64i.p, B.val32i.p);
   EDG_CUDA(cudaGetLastError());
   EDG_CUDA(cudaStreamSynchronize(st));
-  // the complex H x v gathers straight from this table; the SELL layouts serve the real kernels
-  return s->cplx ? EDG_OK : build_sell(s, B);
+  return build_sell(s, B, spin == 1);
 }
 
 // Proper edge colouring of a bipartite multigraph (left: lanes [0,G), right: banks [0,M))
@@ -461,14 +461,11 @@ static int edge_colour(int G, int M, const std::vector<std::pair<int, int>>& edg
 // columns from M = G bank groups (column src sits in group src % M). Per slice and lane
 // group, lanes x groups are edge-coloured; colour = slot. Lanes without an entry in a slot
 // read one of the zero columns DimUp..DimUp+31 whose bank group is free in that slot.
-// Slot c of lane l sits at c*32 + l of its slice, or, with v4, at (c/4)*128 + l*4 + c%4: a
-// lane's slots 4i..4i+3 side by side, one 16-byte load (widths are multiples of 8).
+// Slot c of lane l sits at c*32 + l of its slice.
 static void build_schedule(int64_t dim, int rt, const std::vector<uint32_t>& off, const std::vector<uint32_t>& src,
                            const std::vector<uint32_t>& sgn, std::vector<uint32_t>& soff, std::vector<uint32_t>& ent,
-                           bool* ok, int round_to = kSellBatch, bool v4 = false) {
-  auto at = [v4](int c, int lane) -> size_t {
-    return v4 ? size_t(c / 4) * 128 + size_t(lane) * 4 + size_t(c % 4) : size_t(c) * 32 + size_t(lane);
-  };
+                           bool* ok, int round_to = kSellBatch) {
+  auto at = [](int c, int lane) { return size_t(c) * 32 + size_t(lane); };
   const int G = 32 / rt, M = G;
   const int64_t nsl = (dim + 31) / 32;
   soff.assign(nsl + 1, 0);
@@ -519,6 +516,162 @@ static void build_schedule(int64_t dim, int rt, const std::vector<uint32_t>& off
       }
     }
   }
+}
+
+// 16-bit slot schedule of the tile kernels (SpinBasis::t16_*): a 16-byte shared-memory load of a
+// warp is served 8 lanes at a time, and the 8 are served in one wavefront when their slots fall
+// in distinct 16-byte bank groups (slot % 8) or are the same slot. So each group of 8 columns of
+// a slice is scheduled on its own, and lanes with nothing to do in a slot read a zero slot of
+// a bank group that none of the 8 uses there.
+//  * ordered: each column's sources stay ascending; a lane whose next source clashes waits.
+//    Lanes with the most sources left go first. 23.3 slots for 17.1 hops on the 4x4
+//    half-filled sector (25.0 at the widest group of a slice), where unscheduled source order
+//    takes 39.1 wavefronts; XOR and multiplicative slot hashes and other groupings of the 32
+//    columns gave no fewer.
+//  * any order: an edge colouring of lanes x bank groups, 20.8 slots.
+// Entries are stored in batches of eight slots; a slice ends at a half batch.
+static bool schedule16(int64_t dim, bool ordered, const std::vector<uint32_t>& off, const std::vector<uint32_t>& src,
+                       const std::vector<uint8_t>& code, bool signs, std::vector<uint32_t>& soff,
+                       std::vector<uint16_t>& ent, std::vector<uint8_t>* codes) {
+  constexpr int G = 8;
+  const int64_t nsl = (dim + 31) / 32;
+  soff.assign(nsl, 0);
+  ent.clear();
+  if (codes) codes->clear();
+  std::vector<std::pair<int, int>> edges;
+  std::vector<int> eidx, colour;
+  std::vector<int> slot;  // [slot][lane]: table index, -1 when idle
+  size_t nent = 0;
+  for (int64_t sl = 0; sl < nsl; ++sl) {
+    slot.clear();
+    size_t width = 1;
+    for (int g = 0; g < 32 / G; ++g) {
+      uint32_t pos[G], end[G];
+      size_t left = 0;
+      for (int l = 0; l < G; ++l) {
+        const int64_t r = sl * 32 + g * G + l;
+        pos[l] = r < dim ? off[r] : 0;
+        end[l] = r < dim ? off[r + 1] : 0;
+        left += end[l] - pos[l];
+      }
+      if (ordered) {
+        int ord[G];
+        for (int l = 0; l < G; ++l) ord[l] = l;
+        for (size_t c = 0; left; ++c) {
+          for (int i = 1; i < G; ++i)  // most sources left first (nearly sorted from slot to slot)
+            for (int j = i; j > 0 && end[ord[j]] - pos[ord[j]] > end[ord[j - 1]] - pos[ord[j - 1]]; --j)
+              std::swap(ord[j], ord[j - 1]);
+          int64_t used[G];
+          std::fill(used, used + G, int64_t(-1));
+          if (slot.size() < (c + 1) * 32) slot.resize((c + 1) * 32, -1);
+          for (int q = 0; q < G; ++q) {
+            const int l = ord[q];
+            if (pos[l] == end[l]) break;
+            const int64_t x = src[pos[l]];
+            if (used[x % G] < 0 || used[x % G] == x) {
+              used[x % G] = x;
+              slot[c * 32 + g * G + l] = int(pos[l]++);
+              --left;
+            }
+          }
+          width = std::max(width, c + 1);
+        }
+      } else {
+        edges.clear();
+        eidx.clear();
+        for (int l = 0; l < G; ++l)
+          for (uint32_t k = pos[l]; k < end[l]; ++k) {
+            edges.push_back({l, int(src[k] % G)});
+            eidx.push_back(int(k));
+          }
+        const int D = edge_colour(G, G, edges, colour);
+        if (D < 0) return false;
+        if (slot.size() < size_t(D) * 32) slot.resize(size_t(D) * 32, -1);
+        for (size_t i = 0; i < edges.size(); ++i) slot[size_t(colour[i]) * 32 + g * G + edges[i].first] = eidx[i];
+        width = std::max(width, size_t(D));
+      }
+    }
+    const size_t nb = (width + 7) / 8;
+    const uint32_t half = uint32_t((width + 3) / 4);
+    if (half > 255) return false;
+    soff[sl] = uint32_t(nent / 256) << 9 | half;
+    slot.resize(nb * 256, -1);
+    ent.resize(nent + nb * 256);
+    if (codes) codes->resize(nent + nb * 256, 0);
+    for (size_t c = 0; c < nb * 8; ++c)
+      for (int g = 0; g < 32 / G; ++g) {
+        const int* s = slot.data() + c * 32 + g * G;
+        unsigned used = 0;
+        for (int l = 0; l < G; ++l)
+          if (s[l] >= 0) used |= 1u << (src[s[l]] % G);
+        int fr = 0;
+        while (fr < G - 1 && ((used >> fr) & 1u)) ++fr;
+        const uint32_t zero = uint32_t(dim) + uint32_t((fr - int(dim % G) + G) % G);
+        for (int l = 0; l < G; ++l) {
+          const int k = s[l];
+          const size_t at = nent + (c / 8) * 256 + size_t(g * G + l) * 8 + c % 8;
+          ent[at] = uint16_t(k >= 0 ? src[k] | (signs ? uint32_t(code[k]) << 15 : 0u) : zero);
+          if (codes && k >= 0) (*codes)[at] = code[k];
+        }
+      }
+    nent += nb * 256;
+  }
+  return true;
+}
+
+// Uploads the 16-bit schedules of one spin's hop table (val: values, vi: imaginary parts or
+// empty). Leaves B.t16 false where the tile kernels do not apply: rows whose slots exceed
+// shared memory, or more than 256 distinct values.
+int build_t16(edg_sector_s* s, SpinBasis& B, const std::vector<uint32_t>& off, const std::vector<uint32_t>& src,
+              const std::vector<double>& val, const std::vector<double>& vi) {
+  cudaStream_t st = s->stream;
+  B.t16 = false;
+  B.t16_npal = 0;
+  const int64_t dim = B.dim;
+  if (dim < 1 || tile_smem(dim, 0, 0, 0) > kTileSmemMax) return EDG_OK;
+  std::vector<uint8_t> code(B.nnz + 1, 0);
+  std::vector<double> pal;
+  const bool uniform = vi.empty() && B.sell_uniform;
+  if (uniform) {
+    for (int64_t k = 0; k < B.nnz; ++k) code[k] = val[k] == B.sell_h ? 0 : 1;
+  } else {
+    std::map<std::pair<double, double>, int> seen;
+    for (int64_t k = 0; k < B.nnz; ++k) {
+      const std::pair<double, double> v(val[k], vi.empty() ? 0.0 : vi[k]);
+      auto it = seen.find(v);
+      if (it == seen.end()) {
+        if (seen.size() == 256) return EDG_OK;
+        it = seen.emplace(v, int(seen.size())).first;
+        pal.push_back(v.first);
+        if (!vi.empty()) pal.push_back(v.second);
+      }
+      code[k] = uint8_t(it->second);
+    }
+    if (seen.empty()) pal.assign(vi.empty() ? 1 : 2, 0.0);
+    B.t16_npal = int(std::max<size_t>(1, seen.size()));
+    if (tile_smem(dim, B.t16_npal, 0, vi.empty() ? 8 : 16) > kTileSmemMax) return EDG_OK;
+  }
+  auto up = [&](void* d, const void* h, size_t bytes) { return cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, st); };
+  std::vector<uint32_t> soff;
+  std::vector<uint16_t> ent;
+  std::vector<uint8_t> codes;
+  for (int o = 0; o < (uniform ? 2 : 1); ++o) {
+    if (!schedule16(dim, o == 0, off, src, code, uniform, soff, ent, uniform ? nullptr : &codes)) return EDG_OK;
+    EDG_CHECK(B.t16_off[o].alloc(soff.size(), st, "slot schedule"));
+    EDG_CHECK(B.t16_ent[o].alloc(ent.size(), st, "slot schedule"));
+    EDG_CUDA(up(B.t16_off[o].p, soff.data(), soff.size() * sizeof(uint32_t)));
+    EDG_CUDA(up(B.t16_ent[o].p, ent.data(), ent.size() * sizeof(uint16_t)));
+    EDG_CUDA(cudaStreamSynchronize(st));  // the host vectors are reused
+  }
+  if (!uniform) {
+    EDG_CHECK(B.t16_code.alloc(codes.size(), st, "slot schedule"));
+    EDG_CHECK(B.t16_pal.alloc(pal.size(), st, "slot schedule"));
+    EDG_CUDA(up(B.t16_code.p, codes.data(), codes.size()));
+    EDG_CUDA(up(B.t16_pal.p, pal.data(), pal.size() * sizeof(double)));
+    EDG_CUDA(cudaStreamSynchronize(st));
+  }
+  B.t16 = true;
+  return EDG_OK;
 }
 
 // Kronecker split of one spin's gather table at bit m (SpinBasis::kron_*), planned on the
@@ -898,9 +1051,11 @@ int build_variants(edg_sector_s* s, SpinBasis& B) {
   return EDG_OK;
 }
 
-// SELL-32 copy of a gather table, built on the host from the device CSR (the tables are
-// O(DimUp) -- about 1 MB for a 4x4 lattice -- so this is a one-off of milliseconds).
-int build_sell(edg_sector_s* s, SpinBasis& B) {
+// Work split of the down pass and, for the up spin, the schedules of the up pass: the tile
+// kernels' 16-bit slots or, for rows and tables those do not take, the SELL-32 copy. Built on the
+// host from the device CSR (the tables are O(DimUp), about 1 MB for a 4x4 lattice, so this is a
+// one-off of milliseconds).
+int build_sell(edg_sector_s* s, SpinBasis& B, bool up) {
   cudaStream_t st = s->stream;
   const int64_t dim = B.dim;
   std::vector<uint32_t> off(dim + 1), src(B.nnz + 1);
@@ -952,6 +1107,22 @@ int build_sell(edg_sector_s* s, SpinBasis& B) {
     EDG_CUDA(cudaMemcpyAsync(B.group_rows.p, grows.data(), grows.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
     EDG_CUDA(cudaStreamSynchronize(st));
   }
+  double h0 = B.nnz ? std::fabs(val[0]) : 0.0;
+  bool uniform = true;
+  for (int64_t k = 0; k < B.nnz; ++k)
+    if (std::fabs(val[k]) != h0) { uniform = false; break; }
+  const double hsgn = B.nnz ? (val[0] < 0 ? -h0 : h0) : 0.0;  // value encoded by code 0
+  B.sell_uniform = uniform;
+  B.sell_h = hsgn;
+  if (!up) return EDG_OK;
+  std::vector<double> vi;
+  if (s->cplx) {
+    vi.resize(B.nnz + 1);
+    if (B.nnz) EDG_CUDA(cudaMemcpyAsync(vi.data(), B.val64i.p, B.nnz * sizeof(double), cudaMemcpyDeviceToHost, st));
+    EDG_CUDA(cudaStreamSynchronize(st));
+  }
+  EDG_CHECK(build_t16(s, B, off, src, val, vi));
+  if (B.t16 || s->cplx) return EDG_OK;
   std::vector<uint32_t> soff(nsl + 1, 0);
   for (int64_t sl = 0; sl < nsl; ++sl) {
     uint32_t w = 0;
@@ -959,11 +1130,6 @@ int build_sell(edg_sector_s* s, SpinBasis& B) {
     w = (w + kSellBatch - 1) / kSellBatch * kSellBatch;
     soff[sl + 1] = soff[sl] + 32 * w;
   }
-  double h0 = B.nnz ? std::fabs(val[0]) : 0.0;
-  bool uniform = true;
-  for (int64_t k = 0; k < B.nnz; ++k)
-    if (std::fabs(val[k]) != h0) { uniform = false; break; }
-  const double hsgn = B.nnz ? (val[0] < 0 ? -h0 : h0) : 0.0;  // value encoded by code 0
   // entry: bit 31 = sign (uniform tables), bits 0..30 = source; padding points at the
   // zero slot dim that the up pass keeps after the staged rows
   std::vector<uint32_t> ent(soff[nsl] + 1, uint32_t(dim));
@@ -979,11 +1145,8 @@ int build_sell(edg_sector_s* s, SpinBasis& B) {
       ent[pos] = src[e] | (sign << 31);
     }
   }
-  B.sell_uniform = uniform;
-  B.sell_h = hsgn;
   // FP32 conflict-free schedule (uniform tables whose rows fit the shared-memory up pass)
   B.sched_rt = 0;
-  B.sched_v4 = false;
   B.sched_ent.reset();
   B.sched_off.reset();
   const int rt32 = up_rows_per_cta(dim, sizeof(float));
@@ -992,11 +1155,8 @@ int build_sell(edg_sector_s* s, SpinBasis& B) {
     for (int64_t k = 0; k < B.nnz; ++k) sg[k] = (val[k] == hsgn) ? 0u : 1u;
     std::vector<uint32_t> qoff, qent;
     bool ok = false;
-    // the two-CTA form of the up pass loads its entries four slots at a time
-    const bool v4 = size_t(dim + kUpZeroSlots) * rt32 * sizeof(float) <= kUpSmemTwoPerSM;
-    build_schedule(dim, rt32, off, src, sg, qoff, qent, &ok, kSellBatch, v4);
+    build_schedule(dim, rt32, off, src, sg, qoff, qent, &ok);
     if (ok) {
-      B.sched_v4 = v4;
       qent.push_back(uint32_t(dim));
       EDG_CHECK(B.sched_off.alloc(qoff.size(), st, "SELL schedule"));
       EDG_CHECK(B.sched_ent.alloc(qent.size(), st, "SELL schedule"));

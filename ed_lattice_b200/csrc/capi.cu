@@ -228,11 +228,12 @@ int edg_sector_create(const edg_model* m, int nup, int ndw, int form, edg_sector
     edg_sector_destroy(s);
     return st;
   }
-  // Default H x v of a small real stored sector: the single pass (down-pass choice 3), whose
-  // vectors sit in L2; from about 500,000 states up the two-pass kernels win (measured on the
-  // 3x4 and 4x4 lattices: 0.0085 against 0.0146 ms FP64 at D = 48,400, 0.0515 against 0.0474
-  // at D = 853,776). edg_sector_autotune and edg_sector_set_kernels override it.
-  if (!s->cplx && s->form == EDG_FORM_STORED && s->dim <= kFusedMaxDim) s->hxv_dw[0] = s->hxv_dw[1] = 3;
+  // Default H x v of a real stored sector whose vectors sit in L2: the single pass (down-pass
+  // choice 3). edg_sector_autotune and edg_sector_set_kernels override it.
+  if (!s->cplx && s->form == EDG_FORM_STORED) {
+    if (s->dim <= kFusedMaxDim64) s->hxv_dw[0] = 3;
+    if (s->dim <= kFusedMaxDim32) s->hxv_dw[1] = 3;
+  }
   *out = s;
   return EDG_OK;
 }

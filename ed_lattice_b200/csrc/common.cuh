@@ -154,7 +154,6 @@ struct SpinBasis {
   DevBuf<uint32_t> sched_ent;
   DevBuf<uint32_t> sched_off;
   int sched_rt = 0;             // rows-per-CTA of the FP32 up pass the schedule was built for
-  bool sched_v4 = false;        // slots stored four per lane together (two 16-byte loads per batch)
   // Packed FP32 schedule (uniform tables, 2 * (DimUp + 32) <= 32768 slots): the conflict-free
   // slot schedule for two rows per CTA with slot counts rounded to 2 instead of 8, two 16-bit
   // entries per 32-bit word (entry 2k of a row in the low half of word k, 2k+1 in the high
@@ -165,6 +164,19 @@ struct SpinBasis {
   DevBuf<uint32_t> p16_off;     // [nslices+1] word offsets, multiples of 32
   DevBuf<uint32_t> p16f_ent;    // the same words with the sign as bit 15 of each entry
   uint32_t p16_negoff = 0;      // 0: no packed schedule
+  // 16-bit slot schedule of the tile kernels (tile.cu), for rows whose 16-byte slots fit in
+  // shared memory: [0] keeps each row's sources ascending (FP64, complex), [1] any order
+  // (FP32, uniform tables). Entry: bits 0..14 the shared-memory slot of the source (DimUp +
+  // 0..7: a zero slot), bit 15 the sign of the uniform value. A batch is eight slots, lane l's
+  // eight entries side by side (one 16-byte load); t16_off holds each slice's first half
+  // batch (a slice starts at a whole batch) << 8 | its half batches. Tables of more than one |value| keep a
+  // palette of at most 256 values instead of the sign, one 8-bit code per entry.
+  bool t16 = false;
+  DevBuf<uint16_t> t16_ent[2];
+  DevBuf<uint32_t> t16_off[2];  // [nslices]
+  DevBuf<uint8_t> t16_code;     // codes of the order-keeping schedule
+  DevBuf<double> t16_pal;       // [npal], or [npal][2] (complex Hij)
+  int t16_npal = 0;             // 0: uniform
   // Column-split copy of the SELL table for rows too long to stage whole in shared memory
   // (FP64 rows above 227 KB): part p lists, per slice, the entries whose source lies in
   // columns [split_col[p], split_col[p+1]), stored as source - split_col[p] (padding: the
@@ -224,7 +236,18 @@ struct SpinBasis {
   DevBuf<uint32_t> kron_xwid;     // per warp and step (stride kron_lmax): slots
 };
 
-constexpr int64_t kFusedMaxDim = 500000;  // largest sector that defaults to the single-pass H x v
+// Largest sector that defaults to the single-pass H x v, FP64 and FP32: its source rows must
+// come from L2, and the two-pass kernels' down pass, which sweeps L2-sized column slabs, wins
+// beyond. Measured (us, single pass against two passes): FP64 24.6/43.2 at D = 853,776, 183/215
+// at 10,306,296, 152/162 at 7,949,760, 399/386 at 19,079,424; FP32 17.4/28.8, 32.6/37.0 at
+// 2,944,656, 94/84 at 7,949,760, 247/216 at 19,079,424.
+constexpr int64_t kFusedMaxDim64 = 12000000, kFusedMaxDim32 = 4000000;
+// Complex sectors, either precision (us, one launch against two passes: complex128 326/443 at
+// 7,949,760, 342/463 at 9,018,009).
+constexpr int64_t kFusedMaxDimC = 10000000;
+// Smallest sector whose single pass runs by row tiles (tile.cu): below, the tiles are too few
+// and the per-column gathers of k_hxv_fused finish sooner.
+constexpr int64_t kTileMinDim = 20000;
 constexpr int kKronThreads = 512;  // threads per CTA of the Kronecker up pass
 constexpr int kKronLL = 12;        // LL entries per low part held in registers
 // Shared memory of the Kronecker up pass: rt staged rows plus the zero slots, then the block
@@ -289,14 +312,16 @@ struct edg_sector_s {
   // (two CTAs per SM), 3 = single pass (k_hxv_fused: the whole H x v, no up pass); up pass
   // (FP32) 0 = 32-bit SELL schedule, 1 = packed 16-bit schedule with negated copies, 2 = packed
   // 16-bit schedule with sign bits, 3 = Kronecker schedule. Until tuned: 3/0 for real stored
-  // sectors of at most kFusedMaxDim states, else 0/0.
+  // sectors of at most kFusedMaxDim64 / kFusedMaxDim32 states, else 0/0.
   int hxv_dw[2] = {0, 0};
   int hxv_up[2] = {0, 0};
 };
 
 namespace edg {
 
-// Rows per CTA of the shared-memory up pass for element size `elem` (4 or 8 bytes): four FP32
+// Rows per CTA of the SELL up pass (k_up_smem: the rows and tables that the tile kernels do not
+// take, and the staging of the packed and Kronecker passes) for element size `elem` (4 or 8
+// bytes): four FP32
 // rows if they fit two CTAs per SM (113 KB each), else two rows (two CTAs per SM if they fit,
 // else one CTA of up to 227 KB), else one row with one CTA per SM, else 0 (the row does not
 // fit; the L1-gather kernel takes over). On the 4x4 half-filled sector (DimUp 12870): FP32
@@ -306,6 +331,14 @@ namespace edg {
 constexpr size_t kUpSmemTwoPerSM = 113 * 1024;
 constexpr size_t kUpSmemOnePerSM = 227 * 1024;
 constexpr int kUpZeroSlots = 32;
+constexpr int kT16Zero = 8;    // zero slots after a tile, one per 16-byte bank group
+// Shared memory of a tile kernel: the slots, `hops` down hops (value and source row) and the
+// palette of `elem`-byte values, the slices' offsets.
+constexpr size_t kTileSmemMax = 226 * 1024;  // leaves room for the kernels' static arrays
+inline size_t tile_smem(int64_t dimup, int npal, int hops, size_t elem) {
+  return size_t(dimup + kT16Zero) * 16 + size_t(hops) * ((elem + sizeof(uint32_t) + 7) / 8 * 8) + size_t(npal) * elem +
+         size_t((dimup + 31) / 32) * sizeof(uint32_t);
+}
 constexpr int kSellBatch = 8;  // SELL slice widths are multiples of this (entries loaded per batch)
 inline int up_rows_per_cta(int64_t dimup, size_t elem) {
   const size_t row = size_t(dimup + kUpZeroSlots) * elem;
@@ -346,14 +379,20 @@ template <typename T>
 int hxv_block_lz(edg_sector_s* s, int ncols, const int* active, const T* u, const T* uprev, T* w, const double* bn,
                  int64_t sstride, int j, double* partial, double* aout);
 
+// ---- tile.cu
+// Whether the tile kernels take this sector's vectors (elem bytes per element), for the up pass
+// alone or (down) the whole product.
+bool tile_available(const edg_sector_s* s, size_t elem, bool down);
+
 // ---- vecops.cu
 constexpr int kRedBlocks = 592;  // 148 SMs x 4: fixed reduction grid (deterministic sums)
 constexpr int kRedThreads = 256;
-// A reduction scratch holds kRedBlocks partials and, at index kRedBlocks, the arrival counter
+constexpr int kRedMaxBlocks = 148 * 16;  // most blocks of any fused reduction (the tile kernels')
+// A reduction scratch holds kRedMaxBlocks partials and, at index kRedMaxBlocks, the arrival counter
 // of the fused finish (the last block of a reduction sums the partials and resets it to 0):
 // kRedSlots doubles. The counter must be zero when the scratch is first used
 // (red_scratch_reset).
-constexpr int kRedSlots = kRedBlocks + 2;
+constexpr int kRedSlots = kRedMaxBlocks + 2;
 int red_scratch_reset(cudaStream_t st, double* partial);
 template <typename T>
 int dot_dev(cudaStream_t st, const T* x, const T* y, int64_t n, double* partial, double* out);

@@ -15,76 +15,11 @@
 #include <cstdlib>
 #include <type_traits>
 
-#include "common.cuh"
+#include "hxv.cuh"
 #include "reduce.cuh"
 
 namespace edg {
 namespace {
-
-template <typename T>
-struct HxvArgs {
-  const T* __restrict__ v;
-  T* __restrict__ hv;
-  int64_t dimup, dimdw;
-  const uint32_t* __restrict__ off_up;
-  const uint32_t* __restrict__ src_up;
-  const T* __restrict__ val_up;
-  const uint32_t* __restrict__ off_dw;
-  const uint32_t* __restrict__ src_dw;
-  const T* __restrict__ val_dw;
-  const T* __restrict__ e_up;
-  const T* __restrict__ e_dw;
-  const uint32_t* __restrict__ map_up;
-  const uint32_t* __restrict__ map_dw;
-  T U;
-  // Lanczos-fused mode (v = u / bn[jstep] is applied with the scale folded into the matrix
-  // elements; the step forms w = Hv - (bn[j]/bn[j-1]) uprev and the up pass the partial
-  // <v, w>; lz_sub_in_dw says which pass subtracts uprev)
-  const double* __restrict__ bn = nullptr;
-  int jstep = 0;
-  const T* __restrict__ uprev = nullptr;
-  double* __restrict__ partial = nullptr;  // reduction scratch [kRedSlots]
-  double* __restrict__ red_out = nullptr;  // receives <v, w>
-  // Block mode (several vectors of the sector in one launch, blockIdx.y = column c): column c
-  // reads v + c*vstride, writes hv + c*vstride, uses uprev + c*vstride, bn + c*sstride,
-  // red_out + c*sstride and the scratch partial + c*kRedSlots; a column whose active[c] is 0
-  // is skipped. ncols is the launch's gridDim.y (1 for a single vector).
-  int64_t vstride = 0, sstride = 0;
-  const int* __restrict__ active = nullptr;
-  int ncols = 1;
-  int dwv = 0, upv = 0;  // kernel choice (edg_sector_s::hxv_dw / hxv_up)
-};
-
-// Which pass of the Lanczos-fused step subtracts c * uprev. FP32: the down pass, as the start
-// of its diagonal term (it runs at a fraction of HBM bandwidth, and the up pass, short of
-// registers, then reads no third vector). FP64: the up pass, after all hops, which is the
-// reference's order (w = Hv - b u_prev), so FP64 coefficients stay bit-exact.
-template <typename T>
-constexpr bool lz_sub_in_dw() { return sizeof(T) == 4; }
-
-// Points a block-mode launch's arguments at this CTA's column; false when the column has
-// stopped. A single-vector launch (gridDim.y == 1, active == nullptr) is left as it is.
-template <typename T>
-__device__ __forceinline__ bool select_column(HxvArgs<T>& a) {
-  const int64_t c = blockIdx.y;
-  if (a.active && !a.active[c]) return false;
-  if (c) {
-    a.v += c * a.vstride;
-    a.hv += c * a.vstride;
-    if (a.uprev) a.uprev += c * a.vstride;
-    if (a.bn) a.bn += c * a.sstride;
-    if (a.partial) a.partial += c * kRedSlots;
-    if (a.red_out) a.red_out += c * a.sstride;
-  }
-  return true;
-}
-
-template <typename T>
-__device__ __forceinline__ T fmaT(T a, T b, T c);
-template <>
-__device__ __forceinline__ float fmaT<float>(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-template <>
-__device__ __forceinline__ double fmaT<double>(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // Row pass: one CTA per row idw (grid-stride), threads along iup. H_up gathers hit L1/L2
 // (a row is DimUp*sizeof(T) bytes). FIRST: hv = diag*v + up-part; else hv += up-part.
@@ -115,59 +50,13 @@ __global__ void __launch_bounds__(256) k_up_rows(HxvArgs<T> a) {
 // gathers H_up's sources from there instead of from L1, where random 4-byte reads cost a
 // wavefront per distinct line. The table is SELL-32: the k-th entries of a warp's 32
 // target columns are one coalesced 128-byte read, shared by the RT rows.
-template <typename T, int RT>
-struct VecT;
-template <> struct VecT<float, 1> { using type = float; };
-template <> struct VecT<float, 2> { using type = float2; };
-template <> struct VecT<float, 4> { using type = float4; };
-template <> struct VecT<double, 1> { using type = double; };
-template <> struct VecT<double, 2> { using type = double2; };
-
 template <typename T>
 struct SellArgs {
   const uint32_t* __restrict__ ent;
   const uint32_t* __restrict__ off;
   const T* __restrict__ val;  // non-uniform tables only
   T h;                        // |value| with the sign of code 0 (uniform tables)
-  bool v4 = false;            // a lane's slots stored four together (SpinBasis::sched_v4)
 };
-
-// acc[0..RT) += h * x[0..RT): packed FP32x2 FMAs where the pair shares h (Blackwell
-// fma.rn.f32x2; each lane is an IEEE fma, identical to two scalar ones).
-template <typename T, int RT>
-struct Fma {
-  static __device__ __forceinline__ void run(T h, const T* x, T* acc) {
-#pragma unroll
-    for (int r = 0; r < RT; ++r) acc[r] = fmaT<T>(h, x[r], acc[r]);
-  }
-};
-__device__ __forceinline__ void ffma2(float h, const float* x, float* acc) {
-  uint64_t d;
-  const uint64_t uh = (uint64_t(__float_as_uint(h)) << 32) | __float_as_uint(h);
-  const uint64_t ux = (uint64_t(__float_as_uint(x[1])) << 32) | __float_as_uint(x[0]);
-  const uint64_t ua = (uint64_t(__float_as_uint(acc[1])) << 32) | __float_as_uint(acc[0]);
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(uh), "l"(ux), "l"(ua));
-  acc[0] = __uint_as_float(uint32_t(d));
-  acc[1] = __uint_as_float(uint32_t(d >> 32));
-}
-template <>
-struct Fma<float, 2> {
-  static __device__ __forceinline__ void run(float h, const float* x, float* acc) { ffma2(h, x, acc); }
-};
-template <>
-struct Fma<float, 4> {
-  static __device__ __forceinline__ void run(float h, const float* x, float* acc) {
-    ffma2(h, x, acc);
-    ffma2(h, x + 2, acc + 2);
-  }
-};
-
-__device__ __forceinline__ float flip_sign(float h, uint32_t e) {
-  return __uint_as_float(__float_as_uint(h) ^ (e & 0x80000000u));
-}
-__device__ __forceinline__ double flip_sign(double h, uint32_t e) {
-  return __longlong_as_double(__double_as_longlong(h) ^ (static_cast<long long>(e & 0x80000000u) << 32));
-}
 
 // SELL entry: bit 31 = sign of the uniform value, bits 0..30 = source column (DimUp for
 // padding: a zero slot after the staged rows, so padding needs no branch).
@@ -183,9 +72,7 @@ __device__ __forceinline__ double flip_sign(double h, uint32_t e) {
 template <typename T, bool LZ, bool ONE>
 constexpr int up_threads() { return LZ && !ONE && !lz_sub_in_dw<T>() ? 768 : 1024; }
 
-// E4: the table stores a lane's slots four together (sched_v4), so a batch of 8 entries is
-// two 16-byte loads per lane instead of eight 4-byte ones (two CTAs per SM, uniform tables).
-template <typename T, int RT, bool FIRST, bool UNIFORM, bool LZ, bool ONE, bool E4 = false>
+template <typename T, int RT, bool FIRST, bool UNIFORM, bool LZ, bool ONE>
 __global__ void __launch_bounds__(up_threads<T, LZ, ONE>(), ONE ? 1 : 2) k_up_smem(HxvArgs<T> a, SellArgs<T> sl, int64_t nrowblk) {
   if (!select_column(a)) return;
   using V = typename VecT<T, RT>::type;
@@ -265,18 +152,6 @@ __global__ void __launch_bounds__(up_threads<T, LZ, ONE>(), ONE ? 1 : 2) k_up_sm
           }
 #pragma unroll
           for (int u = 0; u < kUpBatch; ++u) e[u] = en[u];
-        }
-      } else if (E4 && UNIFORM) {
-        static_assert(!E4 || kUpBatch == 8, "two 16-byte entry loads per batch");
-        const uint4* __restrict__ ent4 = reinterpret_cast<const uint4*>(sl.ent);
-        for (uint32_t q = o >> 2; q < (o1 >> 2); q += 8 * kUpBatch) {
-          const uint4 x0 = __ldg(ent4 + q + lane), x1 = __ldg(ent4 + q + 32 + lane);
-          const uint32_t e[kUpBatch] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-#pragma unroll
-          for (int u = 0; u < kUpBatch; ++u) {
-            const V x = S[e[u] & 0x7fffffffu];
-            Fma<T, RT>::run(flip_sign(hs, e[u]), reinterpret_cast<const T*>(&x), acc);
-          }
         }
       } else {
         for (uint32_t p0 = o + lane; p0 < o1; p0 += 32 * kUpBatch) {
@@ -846,9 +721,10 @@ __global__ void __launch_bounds__(256) k_hxv_fused(HxvArgs<T> a, int64_t ntiles)
 // is read once per hop; no global load of the hop list sits in the inner loop.
 constexpr int kDwHops = 32;  // hop-list capacity per row held in shared memory
 
-template <typename T, int VEC, int NSEG, int KU, bool FIRST, bool SCALED>
+template <typename T, int VEC, int NSEG, int KU, bool FIRST, bool SCALED, int W = 1>
 __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t* __restrict__ goff,
-                                                const uint32_t* __restrict__ grows, int64_t nslab) {
+                                                const uint32_t* __restrict__ grows, int64_t nslab,
+                                                const T* __restrict__ vi_dw = nullptr) {
   if (!select_column(a)) return;
   extern __shared__ __align__(16) unsigned char smem_dw[];
   // the Lanczos scale 1/bn[j] (SCALED): folded into the hop values staged below, and read
@@ -865,8 +741,8 @@ __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t*
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const uint32_t gr0 = goff[blockIdx.x];
   const int nr = int(goff[blockIdx.x + 1] - gr0);
-  T* s_val = reinterpret_cast<T*>(smem_dw);            // [nr][kDwHops]
-  T* s_edw = s_val + size_t(nr) * kDwHops;              // [nr]
+  T* s_val = reinterpret_cast<T*>(smem_dw);            // [nr][kDwHops] of W reals
+  T* s_edw = s_val + size_t(nr) * kDwHops * W;          // [nr]
   uint32_t* s_src = reinterpret_cast<uint32_t*>(s_edw + nr);  // [nr][kDwHops]
   uint32_t* s_row = s_src + size_t(nr) * kDwHops;       // [nr]
   uint32_t* s_mdw = s_row + nr;                         // [nr]
@@ -877,7 +753,8 @@ __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t*
     const int cnt = int(a.off_dw[row + 1] - k0);
     if (lane < cnt) {
       s_src[rr * kDwHops + lane] = a.src_dw[k0 + lane];
-      s_val[rr * kDwHops + lane] = SCALED ? T(double(a.val_dw[k0 + lane]) * sc) : a.val_dw[k0 + lane];
+      s_val[(rr * kDwHops + lane) * W] = SCALED ? T(double(a.val_dw[k0 + lane]) * sc) : a.val_dw[k0 + lane];
+      if (W == 2) s_val[(rr * kDwHops + lane) * W + W - 1] = vi_dw[k0 + lane];
     }
     if (lane == 0) {
       s_row[rr] = row;
@@ -887,11 +764,13 @@ __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t*
     }
   }
   const int64_t dimup = a.dimup;
-  constexpr int SEGW = 32 * VEC;  // columns per warp-wide segment
+  static_assert(W == 1 || VEC == 2, "a lane reads one complex element");
+  constexpr int EPL = VEC / W;    // elements per lane
+  constexpr int SEGW = 32 * EPL;  // columns per warp-wide segment
   for (int64_t slab = 0; slab < nslab; ++slab) {
     if (threadIdx.x == 0) s_ctr = 0;
     __syncthreads();
-    const int64_t col0 = slab * (SEGW * NSEG) + int64_t(lane) * VEC;
+    const int64_t col0 = slab * (SEGW * NSEG) + int64_t(lane) * EPL;
     bool act[NSEG];
 #pragma unroll
     for (int g = 0; g < NSEG; ++g) act[g] = col0 + g * SEGW < dimup;
@@ -901,11 +780,11 @@ __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t*
       rr = __shfl_sync(0xffffffffu, rr, 0);
       if (rr >= nr) break;
       const int64_t idw = s_row[rr];
-      const T* __restrict__ vrow0 = a.v + col0;   // + src*dimup per hop
+      const T* __restrict__ vrow0 = a.v + col0 * W;   // + src*dimup*W per hop
       const int64_t e0 = idw * dimup + col0;
       const int cnt = s_cnt[rr];
       const uint32_t* hs = s_src + rr * kDwHops;
-      const T* hvv = s_val + rr * kDwHops;
+      const T* hvv = s_val + rr * kDwHops * W;
       T acc[NSEG][VEC];
 #pragma unroll
       for (int g = 0; g < NSEG; ++g) {
@@ -915,12 +794,13 @@ __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t*
           const T edw = s_edw[rr];
           const uint32_t mdw = s_mdw[rr];
           T x[VEC], up[VEC];
-          VecLd<T, VEC>::load(a.v + e0 + g * SEGW, x);
+          VecLd<T, VEC>::load(a.v + (e0 + g * SEGW) * W, x);
           if (SUB) VecLd<T, VEC>::load(a.uprev + e0 + g * SEGW, up);
           const double scl = SCALED ? *static_cast<volatile double*>(&s_sc) : 1.0;
 #pragma unroll
           for (int r = 0; r < VEC; ++r) {
-            const T d = a.e_up[c + r] + edw + a.U * T(__popc(a.map_up[c + r] & mdw));
+            const int64_t cr = c + r / W;
+            const T d = a.e_up[cr] + edw + a.U * T(__popc(a.map_up[cr] & mdw));
             acc[g][r] = (SCALED ? T(double(d) * scl) : d) * x[r];
           }
           if (SUB) {
@@ -930,7 +810,7 @@ __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t*
           }
         } else {
 #pragma unroll
-          for (int r = 0; r < VEC; ++r) acc[g][r] = a.hv[e0 + g * SEGW + r];
+          for (int r = 0; r < VEC; ++r) acc[g][r] = a.hv[(e0 + g * SEGW) * W + r];
         }
       }
       for (int k = 0; k < cnt; k += KU) {
@@ -938,18 +818,21 @@ __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t*
 #pragma unroll
         for (int u = 0; u < KU; ++u) {
           const int kk = k + u < cnt ? k + u : k;
-          const T* __restrict__ src = vrow0 + int64_t(hs[kk]) * dimup;
+          const T* __restrict__ src = vrow0 + int64_t(hs[kk]) * dimup * W;
 #pragma unroll
           for (int g = 0; g < NSEG; ++g)
-            if (act[g]) VecLd<T, VEC>::load(src + g * SEGW, x[u][g]);
+            if (act[g]) VecLd<T, VEC>::load(src + g * SEGW * W, x[u][g]);
         }
 #pragma unroll
         for (int u = 0; u < KU; ++u) {
           if (k + u < cnt) {
-            const T h = hvv[k + u];
+            const T h = hvv[(k + u) * W], hi = W == 2 ? hvv[(k + u) * W + W - 1] : T(0);
 #pragma unroll
             for (int g = 0; g < NSEG; ++g)
-              if (act[g]) Fma<T, VEC>::run(h, x[u][g], acc[g]);
+              if (act[g]) {
+                if constexpr (W == 1) Fma<T, VEC>::run(h, x[u][g], acc[g]);
+                else cmad(h, hi, x[u][g], acc[g]);
+              }
           }
         }
       }
@@ -957,7 +840,7 @@ __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t*
       for (int g = 0; g < NSEG; ++g)
         if (act[g]) {
 #pragma unroll
-          for (int r = 0; r < VEC; ++r) __stcs(a.hv + e0 + g * SEGW + r, acc[g][r]);
+          for (int r = 0; r < VEC; ++r) __stcs(a.hv + (e0 + g * SEGW) * W + r, acc[g][r]);
         }
     }
     __syncthreads();
@@ -1285,13 +1168,10 @@ struct Cplx<double> {
   using type = double2;
 };
 
-// acc += h * y for complex h = (hr, hi), y
 template <typename T, typename T2>
-__device__ __forceinline__ void cmad(T hr, T hi, T2 y, T& re, T& im) {
-  re = fmaT<T>(hr, y.x, re);
-  re = fmaT<T>(-hi, y.y, re);
-  im = fmaT<T>(hr, y.y, im);
-  im = fmaT<T>(hi, y.x, im);
+__device__ __forceinline__ void cmad2(T hr, T hi, T2 y, T* acc) {
+  const T x[2] = {y.x, y.y};
+  cmad(hr, hi, x, acc);
 }
 
 // Stored form, one thread per element: the diagonal, then the down hops, then the up hops,
@@ -1308,14 +1188,14 @@ __global__ void __launch_bounds__(256) k_cplx_stored(HxvArgs<T> a, const T* __re
     const int64_t idw = e / a.dimup, iup = e - idw * a.dimup;
     const T d = a.e_up[iup] + a.e_dw[idw] + a.U * T(__popc(a.map_up[iup] & a.map_dw[idw]));
     const T2 x = v[e];
-    T re = d * x.x, im = d * x.y;
+    T acc[2] = {d * x.x, d * x.y};
     for (uint32_t k = a.off_dw[idw]; k < a.off_dw[idw + 1]; ++k)
-      cmad(a.val_dw[k], vi_dw[k], v[int64_t(a.src_dw[k]) * a.dimup + iup], re, im);
+      cmad2(a.val_dw[k], vi_dw[k], v[int64_t(a.src_dw[k]) * a.dimup + iup], acc);
     for (uint32_t k = a.off_up[iup]; k < a.off_up[iup + 1]; ++k)
-      cmad(a.val_up[k], vi_up[k], v[idw * a.dimup + a.src_up[k]], re, im);
+      cmad2(a.val_up[k], vi_up[k], v[idw * a.dimup + a.src_up[k]], acc);
     T2 out;
-    out.x = re;
-    out.y = im;
+    out.x = acc[0];
+    out.y = acc[1];
     hv[e] = out;
   }
 }
@@ -1347,13 +1227,13 @@ __global__ void __launch_bounds__(256) k_cplx_direct(HxvArgs<T> a, DirectArgsHdr
     const uint32_t mup = a.map_up[iup], mdw = a.map_dw[idw];
     const T dg = a.e_up[iup] + a.e_dw[idw] + a.U * T(__popc(mup & mdw));
     const T2 x = v[e];
-    T re = dg * x.x, im = dg * x.y;
+    T acc[2] = {dg * x.x, dg * x.y};
     for (int k = 0; k < d.nb_up; ++k) {
       const int ba = sb[2 * k], bb = sb[2 * k + 1];
       if (((mup >> ba) & 1u) && !((mup >> bb) & 1u)) {
         const uint32_t t = (mup & ~(1u << ba)) | (1u << bb);
         const T sg = between_parity_d(mup, ba, bb) ? T(-1) : T(1);
-        cmad(sg * shr[k], sg * shi[k], v[idw * a.dimup + rank_of_d(t, sC)], re, im);
+        cmad2(sg * shr[k], sg * shi[k], v[idw * a.dimup + rank_of_d(t, sC)], acc);
       }
     }
     for (int k = d.nb_up; k < nb; ++k) {
@@ -1361,12 +1241,12 @@ __global__ void __launch_bounds__(256) k_cplx_direct(HxvArgs<T> a, DirectArgsHdr
       if (((mdw >> ba) & 1u) && !((mdw >> bb) & 1u)) {
         const uint32_t t = (mdw & ~(1u << ba)) | (1u << bb);
         const T sg = between_parity_d(mdw, ba, bb) ? T(-1) : T(1);
-        cmad(sg * shr[k], sg * shi[k], v[int64_t(rank_of_d(t, sC)) * a.dimup + iup], re, im);
+        cmad2(sg * shr[k], sg * shi[k], v[int64_t(rank_of_d(t, sC)) * a.dimup + iup], acc);
       }
     }
     T2 out;
-    out.x = re;
-    out.y = im;
+    out.x = acc[0];
+    out.y = acc[1];
     hv[e] = out;
   }
 }
@@ -1401,9 +1281,6 @@ int launch_up_smem(const HxvArgs<T>& a, const SellArgs<T>& sl, cudaStream_t st, 
   const size_t smem = size_t(a.dimup + kUpZeroSlots) * RT * sizeof(T);
   const int per_sm = smem <= kUpSmemTwoPerSM ? 2 : 1;
   auto kern = per_sm == 2 ? k_up_smem<T, RT, FIRST, UNIFORM, LZ, false> : k_up_smem<T, RT, FIRST, UNIFORM, LZ, true>;
-  if constexpr (sizeof(T) == 4 && UNIFORM) {
-    if (per_sm == 2 && sl.v4) kern = k_up_smem<T, RT, FIRST, UNIFORM, LZ, false, true>;
-  }
   if (smem > 48 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   const int64_t nrb = (a.dimdw + RT - 1) / RT;
   int64_t g = nrb < int64_t(sms) * per_sm ? nrb : int64_t(sms) * per_sm;
@@ -1450,7 +1327,7 @@ int dw_pass(const HxvArgs<T>& a, const SpinBasis& Bdw, cudaStream_t st, int sms)
     const size_t smem = size_t(Bdw.group_max) * (kDwHops * (sizeof(T) + 4) + sizeof(T) + 12) + 16;
     if (smem > 48 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     const int64_t nslab = (a.dimup + 32 * vec * NSEG - 1) / (32 * vec * NSEG);
-    kern<<<dim3(Bdw.groups, a.ncols), 256, smem, st>>>(a, Bdw.group_off.p, Bdw.group_rows.p, nslab);
+    kern<<<dim3(Bdw.groups, a.ncols), 256, smem, st>>>(a, Bdw.group_off.p, Bdw.group_rows.p, nslab, nullptr);
     EDG_CUDA(cudaGetLastError());
     return EDG_OK;
   }
@@ -1464,6 +1341,19 @@ int dw_pass(const HxvArgs<T>& a, const SpinBasis& Bdw, cudaStream_t st, int sms)
   const int g = int(want < int64_t(sms) * 8 ? want : int64_t(sms) * 8);
   if (v2) k_dw_seg<T, 2, FIRST><<<g, 256, 0, st>>>(a, ntiles);
   else k_dw_seg<T, 1, FIRST><<<g, 256, 0, st>>>(a, ntiles);
+  EDG_CUDA(cudaGetLastError());
+  return EDG_OK;
+}
+
+// diag*v and the down hops of a complex sector (k_dw_grp on complex elements).
+template <typename T>
+int dw_pass_c(const HxvArgs<T>& a, const SpinBasis& Bdw, const T* vi_dw, cudaStream_t st) {
+  constexpr int NSEG = sizeof(T) == 4 ? 4 : 2, KU = sizeof(T) == 4 ? 3 : 4;
+  auto kern = k_dw_grp<T, 2, NSEG, KU, true, false, 2>;
+  const size_t smem = size_t(Bdw.group_max) * (kDwHops * (2 * sizeof(T) + 4) + sizeof(T) + 12) + 16;
+  if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  const int64_t nslab = (a.dimup + 32 * NSEG - 1) / (32 * NSEG);
+  kern<<<dim3(Bdw.groups, 1), 256, smem, st>>>(a, Bdw.group_off.p, Bdw.group_rows.p, nslab, vi_dw);
   EDG_CUDA(cudaGetLastError());
   return EDG_OK;
 }
@@ -1542,12 +1432,14 @@ bool launch_up_kron(const HxvArgs<float>& a, const SpinBasis& B, cudaStream_t st
 }
 
 template <typename T, bool FIRST, bool LZ>
-int up_pass(const HxvArgs<T>& a, const SpinBasis& B, cudaStream_t st, int sms, int* grid) {
+int up_pass(const HxvArgs<T>& a, edg_sector_s* s, cudaStream_t st, int sms, int* grid) {
+  const SpinBasis& B = s->up;
   if constexpr (std::is_same<T, float>::value && !FIRST) {
     int status = EDG_OK;
     if (launch_up_kron<LZ>(a, B, st, sms, &status)) return status;
     if (launch_up_p16<LZ>(a, B, st, sms, &status)) return status;
   }
+  if (!FIRST && tile_available(s, sizeof(T), false)) return tile_real<T>(a, B, s->dw, false, LZ, st, sms);
   const int rt = up_rows_per_cta(a.dimup, sizeof(T));
   if (rt == 0) {
     if (LZ || a.ncols > 1) {
@@ -1584,14 +1476,14 @@ int up_pass(const HxvArgs<T>& a, const SpinBasis& B, cudaStream_t st, int sms, i
   if (sizeof(T) == 4 && B.sched_rt == rt && B.sched_ent.p) {  // FP32: bank-conflict-free order
     sl.ent = B.sched_ent.p;
     sl.off = B.sched_off.p;
-    sl.v4 = B.sched_v4;
   }
   sl.val = pick_sell<T>(B);
   sl.h = T(B.sell_h);
   constexpr int R4 = sizeof(T) == 4 ? 4 : 2;
-  if (B.sell_uniform) {
-    if (rt == 4) return launch_up_smem<T, R4, FIRST, true, LZ>(a, sl, st, sms, grid);
-    if (rt == 2) return launch_up_smem<T, 2, FIRST, true, LZ>(a, sl, st, sms, grid);
+  if (B.sell_uniform) {  // rows longer than the tile kernels take: two FP32 rows or one at most
+    if constexpr (sizeof(T) == 4) {
+      if (rt == 2) return launch_up_smem<T, 2, FIRST, true, LZ>(a, sl, st, sms, grid);
+    }
     return launch_up_smem<T, 1, FIRST, true, LZ>(a, sl, st, sms, grid);
   }
   if (rt == 4) return launch_up_smem<T, R4, FIRST, false, LZ>(a, sl, st, sms, grid);
@@ -1623,8 +1515,11 @@ HxvArgs<T> make_args(edg_sector_s* s, const T* v, T* hv) {
 }
 
 // Single-pass H x v (down-pass choice 3): one launch does the whole H x v; no up pass.
+// By row tiles (tile.cu) where the tile kernels apply, else the per-column gathers.
 template <typename T, bool LZ>
-int fused_pass(const HxvArgs<T>& a, cudaStream_t st, int sms) {
+int fused_pass(edg_sector_s* s, const HxvArgs<T>& a, cudaStream_t st, int sms) {
+  if (tile_available(s, sizeof(T), true) && s->dim >= kTileMinDim)
+    return tile_real<T>(a, s->up, s->dw, true, LZ, st, sms);
   const int64_t ntiles = a.dimdw * ((a.dimup + 31) / 32);
   const int64_t want = (ntiles + 7) / 8;
   int64_t g = want < int64_t(sms) * 8 ? want : int64_t(sms) * 8;
@@ -1647,6 +1542,16 @@ int hxv_apply(edg_sector_s* s, const T* v, T* hv) {
     const int64_t want = (n + 255) / 256;
     const int g = int(want < int64_t(sms) * 8 ? (want < 1 ? 1 : want) : int64_t(sms) * 8);
     if (s->form == EDG_FORM_STORED) {
+      const T* vi = pick<T>(s->dw.val64i, s->dw.val32i);
+      // the tile kernels, in one launch while the source rows come from L2, else after the
+      // down pass over L2-sized column slabs
+      const bool vec = reinterpret_cast<uintptr_t>(v) % (2 * sizeof(T)) == 0 && reinterpret_cast<uintptr_t>(hv) % (2 * sizeof(T)) == 0;
+      if (vec && s->dim <= kFusedMaxDimC && tile_available(s, 2 * sizeof(T), true))
+        return tile_cplx<T>(a, s->up, s->dw, vi, true, st, sms);
+      if (vec && s->dw.max_row <= kDwHops && s->dw.groups > 0 && tile_available(s, 2 * sizeof(T), false)) {
+        EDG_CHECK(dw_pass_c<T>(a, s->dw, vi, st));
+        return tile_cplx<T>(a, s->up, s->dw, nullptr, false, st, sms);
+      }
       k_cplx_stored<T><<<g, 256, 0, st>>>(a, pick<T>(s->up.val64i, s->up.val32i), pick<T>(s->dw.val64i, s->dw.val32i));
     } else {
       DirectArgsHdr d;
@@ -1665,9 +1570,9 @@ int hxv_apply(edg_sector_s* s, const T* v, T* hv) {
     return EDG_OK;
   }
   if (s->form == EDG_FORM_STORED) {
-    if (a.dwv == 3) return fused_pass<T, false>(a, st, sms);
+    if (a.dwv == 3) return fused_pass<T, false>(s, a, st, sms);
     EDG_CHECK((dw_pass<T, true, false>(a, s->dw, st, sms)));
-    EDG_CHECK((up_pass<T, false, false>(a, s->up, st, sms, nullptr)));
+    EDG_CHECK((up_pass<T, false, false>(a, s, st, sms, nullptr)));
   } else {
     DirectArgsHdr d;
     d.nb_up = s->bonds[0].nb;
@@ -1729,7 +1634,7 @@ int hxv_rows(edg_sector_s* s, int64_t row0, int64_t nrows, const T* v, T* hv) {
   a.dimdw = nrows;
   a.e_dw += row0;
   a.map_dw += row0;
-  return up_pass<T, false, false>(a, s->up, s->stream, sm_count(), nullptr);
+  return up_pass<T, false, false>(a, s, s->stream, sm_count(), nullptr);
 }
 template int hxv_cols<float>(edg_sector_s*, int64_t, int64_t, const float*, float*);
 template int hxv_cols<double>(edg_sector_s*, int64_t, int64_t, const double*, double*);
@@ -1754,9 +1659,9 @@ int hxv_apply_lz(edg_sector_s* s, const T* u, const T* uprev, T* w, const double
   a.partial = partial;
   a.red_out = aout;
   const int sms = sm_count();
-  if (a.dwv == 3) return fused_pass<T, true>(a, s->stream, sms);
+  if (a.dwv == 3) return fused_pass<T, true>(s, a, s->stream, sms);
   EDG_CHECK((dw_pass<T, true, true>(a, s->dw, s->stream, sms)));
-  EDG_CHECK((up_pass<T, false, true>(a, s->up, s->stream, sms, nullptr)));
+  EDG_CHECK((up_pass<T, false, true>(a, s, s->stream, sms, nullptr)));
   return EDG_OK;
 }
 bool hxv_lz_available(const edg_sector_s* s, size_t elem) {
@@ -1774,9 +1679,9 @@ int hxv_block(edg_sector_s* s, int ncols, const int* active, const T* v, T* hv) 
   a.active = active;
   a.ncols = ncols;
   const int sms = sm_count();
-  if (a.dwv == 3) return fused_pass<T, false>(a, s->stream, sms);
+  if (a.dwv == 3) return fused_pass<T, false>(s, a, s->stream, sms);
   EDG_CHECK((dw_pass<T, true, false>(a, s->dw, s->stream, sms)));
-  EDG_CHECK((up_pass<T, false, false>(a, s->up, s->stream, sms, nullptr)));
+  EDG_CHECK((up_pass<T, false, false>(a, s, s->stream, sms, nullptr)));
   return EDG_OK;
 }
 
@@ -1798,9 +1703,9 @@ int hxv_block_lz(edg_sector_s* s, int ncols, const int* active, const T* u, cons
   a.active = active;
   a.ncols = ncols;
   const int sms = sm_count();
-  if (a.dwv == 3) return fused_pass<T, true>(a, s->stream, sms);
+  if (a.dwv == 3) return fused_pass<T, true>(s, a, s->stream, sms);
   EDG_CHECK((dw_pass<T, true, true>(a, s->dw, s->stream, sms)));
-  EDG_CHECK((up_pass<T, false, true>(a, s->up, s->stream, sms, nullptr)));
+  EDG_CHECK((up_pass<T, false, true>(a, s, s->stream, sms, nullptr)));
   return EDG_OK;
 }
 // Autotuner: every down-pass x up-pass pair (4 x 4 for FP32, 4 x 1 for FP64; a pair whose

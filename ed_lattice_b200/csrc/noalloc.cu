@@ -30,7 +30,7 @@ namespace {
 
 constexpr int64_t kNoAllocMaxDim = int64_t(1) << 20;
 constexpr int kNoAllocMaxLanc = 1024;
-constexpr int64_t kNoAllocScalars = 4096;  // reduction scratch [kRedSlots] + a [cap] + b [cap+1] + slots
+constexpr int64_t kNoAllocScalars = 8192;  // reduction scratch [kRedSlots] + a [cap] + b [cap+1] + slots
 static_assert(kRedSlots + 2 * (kNoAllocMaxLanc + 1) + 8 <= kNoAllocScalars, "scalar area too small");
 
 // The scratch: [V | P | W] vectors of kNoAllocMaxDim doubles, then the scalar area.

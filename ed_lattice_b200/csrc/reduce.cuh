@@ -6,7 +6,7 @@
 namespace edg {
 
 // Fused reduction tail. Thread 0 of every block has written partial[blockIdx.x]; the last
-// block to arrive (counter at partial[kRedBlocks]) sums partial[0..nblk) with its first
+// block to arrive (counter at partial[kRedMaxBlocks]) sums partial[0..nblk) with its first
 // kRedThreads threads in exactly the order of the one-block finishing pass (strided sums,
 // then the warp-shuffle tree), writes *out and resets the counter. One launch per reduction
 // instead of two, with bit-identical results. Every thread of the block must call it.
@@ -14,7 +14,7 @@ __device__ __forceinline__ void finish_in_last_block(double* __restrict__ partia
                                                      int do_sqrt) {
   __shared__ int s_last;
   __shared__ double s_fin[kRedThreads / 32];
-  unsigned int* ctr = reinterpret_cast<unsigned int*>(partial + kRedBlocks);
+  unsigned int* ctr = reinterpret_cast<unsigned int*>(partial + kRedMaxBlocks);
   if (threadIdx.x == 0) {
     __threadfence();  // this block's partial is visible before it is counted
     s_last = atomicAdd(ctr, 1u) == unsigned(nblk) - 1u;

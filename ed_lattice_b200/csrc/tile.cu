@@ -1,0 +1,460 @@
+// tile.cu -- the H x v over row tiles held in shared memory as 16-byte slots.
+//
+// A CTA stages the RT rows idw of a tile (4 FP32, 2 FP64, 2 complex64 or 1 complex128) column
+// by column: slot iup holds the RT values of column iup, so one 16-byte shared load per up hop
+// feeds RT rows. The up hops of 32 consecutive columns (a slice, one per lane) run slot by slot
+// over a 16-bit schedule (SpinBasis::t16_*, schedule16() in basis.cu). Two forms:
+//  * rows in (down == false): hv already holds diag*v and the down hops; hv += (I x H_up) v.
+//    The up pass of large sectors.
+//  * whole product (down == true): the diagonal, then the row's down hops (one list per row,
+//    the same for every lane: coalesced reads of the source rows), then the up hops. One launch
+//    and one write of hv; the source rows come from L2, so it is the H x v of sectors whose
+//    vectors sit there.
+// Both add the terms of an element in the stored form's order (diag, DW, UP; sources
+// ascending), so FP64 results carry the same bits as spMatVec's restatement.
+//
+// What bounds it: the shared-memory data path, 128 bytes per clock and SM. A slot of a slice
+// takes 4 wavefronts (one per 8 lanes) and half a wavefront of entries; in source order without
+// a schedule bank conflicts took 36-39 wavefronts per 8 lanes and 16-17 hops on the 4x4
+// lattice, with it 22-23. Where a tile fills an SM, staging it is next (a fifth of the pass
+// from HBM; the next tile's rows are therefore fetched into L2 ahead).
+// Measured, before (32-bit SELL entries, two FP32 or two FP64 rows) and now, us:
+//   up pass, 4x4 (8,8)  FP32  1025 -> 817     4x4 (7,7) FP64  1862 -> 1294
+//   up pass, 5x3 (7,8)  FP64   570 -> 398     fused Lanczos 4x4 (6,6) FP64  1084 -> 804
+//   whole product, 3x4 (6,6) FP64: two passes 44.0 -> 22.3; 12 Lanczos columns 491 -> 202
+//   complex128 4x4 (5,5): 2433 (one thread per element, L1 gathers) -> 1157 in two passes;
+//   3x4 (6,6) 81 -> 44, 4x4 (4,5) 825 -> 326 in one launch
+#include <algorithm>
+
+#include "hxv.cuh"
+#include "reduce.cuh"
+
+namespace edg {
+namespace {
+
+template <typename T, int W>
+struct TileArgs {
+  const uint4* __restrict__ ent;       // eight 16-bit entries per lane and batch
+  const uint2* __restrict__ code;      // eight palette codes per lane and batch (PAL)
+  const uint32_t* __restrict__ off;    // [nsl] first half batch (four slots) of a slice << 8 | half batches
+  const double* __restrict__ pal;      // palette: W doubles per code (PAL)
+  T h;                                 // value of sign bit 0 (!PAL)
+  int npal = 0;
+  int nsl = 0, ntile = 0;
+  int csplit = 1;                      // column parts of a tile, each its own work item
+  int cap = 0;                         // down hops kept per row (down form)
+  const T* __restrict__ vi_dw = nullptr;  // imaginary parts of the down values (W == 2)
+};
+
+// One element: W reals.
+template <typename T, int W>
+struct alignas(sizeof(T) * W) Elem {
+  T x[W];
+};
+
+// The 16-byte slot at byte offset `at` of the tile and acc += h * slot. The slot is read as
+// two 64-bit halves so that FP32 pairs feed the packed FMA without repacking.
+template <typename T, int W>
+struct SlotAcc;
+template <>
+struct SlotAcc<float, 1> {  // four rows, two packed pairs
+  uint64_t a[2];
+  __device__ __forceinline__ void set(const float* x) {
+    a[0] = (uint64_t(__float_as_uint(x[1])) << 32) | __float_as_uint(x[0]);
+    a[1] = (uint64_t(__float_as_uint(x[3])) << 32) | __float_as_uint(x[2]);
+  }
+  __device__ __forceinline__ float get(int i) const { return __uint_as_float(uint32_t(a[i >> 1] >> (32 * (i & 1)))); }
+  __device__ __forceinline__ void fma(const float* h, ulonglong2 q) {
+    const uint64_t hh = (uint64_t(__float_as_uint(h[0])) << 32) | __float_as_uint(h[0]);
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a[0]) : "l"(hh), "l"(uint64_t(q.x)));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a[1]) : "l"(hh), "l"(uint64_t(q.y)));
+  }
+};
+template <>
+struct SlotAcc<double, 1> {  // two rows
+  double a[2];
+  __device__ __forceinline__ void set(const double* x) { a[0] = x[0], a[1] = x[1]; }
+  __device__ __forceinline__ double get(int i) const { return a[i]; }
+  __device__ __forceinline__ void fma(const double* h, ulonglong2 q) {
+    a[0] = __fma_rn(h[0], __longlong_as_double(q.x), a[0]);
+    a[1] = __fma_rn(h[0], __longlong_as_double(q.y), a[1]);
+  }
+};
+
+template <>
+struct SlotAcc<double, 2> {  // one complex element
+  double a[2];
+  __device__ __forceinline__ void set(const double* x) { a[0] = x[0], a[1] = x[1]; }
+  __device__ __forceinline__ double get(int i) const { return a[i]; }
+  __device__ __forceinline__ void fma(const double* h, ulonglong2 q) {
+    const double x[2] = {__longlong_as_double(q.x), __longlong_as_double(q.y)};
+    cmad(h[0], h[1], x, a);
+  }
+};
+template <>
+struct SlotAcc<float, 2> {  // two rows of one complex element
+  float a[4];
+  __device__ __forceinline__ void set(const float* x) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = x[i];
+  }
+  __device__ __forceinline__ float get(int i) const { return a[i]; }
+  __device__ __forceinline__ void fma(const float* h, ulonglong2 q) {
+    const float x[4] = {__uint_as_float(uint32_t(q.x)), __uint_as_float(uint32_t(q.x >> 32)),
+                        __uint_as_float(uint32_t(q.y)), __uint_as_float(uint32_t(q.y >> 32))};
+    cmad(h[0], h[1], x, a);
+    cmad(h[0], h[1], x + 2, a + 2);
+  }
+};
+
+// acc += h * x of one element
+template <typename T, int W>
+__device__ __forceinline__ void elem_fma(const T* h, const T* x, T* acc) {
+  if constexpr (W == 1) acc[0] = fmaT<T>(h[0], x[0], acc[0]);
+  else cmad(h[0], h[1], x, acc);
+}
+
+// A down hop of a row: the value and the first element of the source row.
+template <typename T, int W>
+struct alignas(8) Hop {
+  T val[W];
+  uint32_t src;
+};
+
+template <typename T, int W, bool DOWN, bool LZ, bool PAL>
+__global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q) {
+  if (!select_column(a)) return;
+  constexpr int RT = 16 / int(sizeof(T) * W);  // rows per tile
+  constexpr int N = RT * W;                    // reals per slot
+  constexpr int KU = 8 / W;                    // down hops in flight
+  // uprev is subtracted here, after all hops, unless the down pass began from -c * uprev
+  constexpr bool SUB = LZ && (DOWN || !lz_sub_in_dw<T>());
+  using E = Elem<T, W>;
+  using H = Hop<T, W>;
+  extern __shared__ __align__(16) unsigned char smem_tile[];
+  const int dimup = int(a.dimup);
+  ulonglong2* S = reinterpret_cast<ulonglong2*>(smem_tile);
+  H* l_hop = reinterpret_cast<H*>(S + dimup + kT16Zero);  // [RT][cap]
+  T* s_pal = reinterpret_cast<T*>(l_hop + RT * q.cap);
+  uint32_t* s_off = reinterpret_cast<uint32_t*>(s_pal + q.npal * W);  // [nsl]
+  __shared__ double s_lz[2];
+  __shared__ T s_edw[RT];
+  __shared__ uint32_t s_mdw[RT];
+  __shared__ int s_cnt[RT];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  double pa = 0.0, sc = 1.0;
+  if (LZ) {
+    sc = 1.0 / a.bn[a.jstep];
+    if (threadIdx.x == 0) {
+      s_lz[0] = sc;
+      s_lz[1] = a.jstep > 0 ? a.bn[a.jstep] / a.bn[a.jstep - 1] : 0.0;
+    }
+  }
+  const T hs = LZ ? T(double(q.h) * sc) : q.h;
+  if (PAL)
+    for (int i = threadIdx.x; i < q.npal * W; i += blockDim.x) s_pal[i] = T(LZ ? q.pal[i] * sc : q.pal[i]);
+  for (int i = threadIdx.x; i < q.nsl; i += blockDim.x) s_off[i] = q.off[i];
+  if (threadIdx.x < kT16Zero) S[dimup + threadIdx.x] = make_ulonglong2(0, 0);
+  const uint32_t sbase = uint32_t(__cvta_generic_to_shared(S));
+  const int nitem = q.ntile * q.csplit;
+  for (int item = blockIdx.x; item < nitem; item += gridDim.x) {
+    const int tile = q.csplit == 1 ? item : item / q.csplit;
+    const int part = item - tile * q.csplit;
+    const int s0 = q.nsl * part / q.csplit, s1 = q.nsl * (part + 1) / q.csplit;
+    const int64_t r0 = int64_t(tile) * RT;
+    const int rows = int(a.dimdw - r0 < RT ? a.dimdw - r0 : RT);
+    const E* __restrict__ vt = reinterpret_cast<const E*>(a.v) + r0 * dimup;
+    E* __restrict__ ht = reinterpret_cast<E*>(a.hv) + r0 * dimup;
+#pragma unroll 7
+    for (int j = threadIdx.x; j < dimup; j += blockDim.x) {
+      ulonglong2 slot = make_ulonglong2(0, 0);
+      E* xs = reinterpret_cast<E*>(&slot);
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+        if (r < rows) xs[r] = vt[r * dimup + j];
+      S[j] = slot;
+    }
+    if (DOWN) {
+#pragma unroll
+      for (int r = 0; r < RT; ++r) {
+        if (r >= rows) break;
+        const uint32_t k0 = a.off_dw[r0 + r], n = a.off_dw[r0 + r + 1] - k0;
+        for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
+          H h;
+          h.val[0] = LZ ? T(double(a.val_dw[k0 + k]) * sc) : a.val_dw[k0 + k];
+          if (W == 2) h.val[W - 1] = q.vi_dw[k0 + k];
+          h.src = a.src_dw[k0 + k] * uint32_t(dimup);
+          l_hop[r * q.cap + k] = h;
+        }
+        if (threadIdx.x == 0) {
+          s_edw[r] = a.e_dw[r0 + r];
+          s_mdw[r] = a.map_dw[r0 + r];
+          s_cnt[r] = int(n);
+        }
+      }
+    }
+    __syncthreads();
+    // The first entries, (rows-in form) sums and (down form) diagonal terms of each slice are
+    // loaded while the slice before it runs.
+    int sl = s0 + warp;
+    uint32_t o = 0, o1 = 0;
+    uint4 b0 = make_uint4(0u, 0u, 0u, 0u);
+    uint2 c0 = make_uint2(0u, 0u);
+    E hn[RT] = {};
+    T eun = T(0);
+    uint32_t mun = 0;
+    if (sl < s1) {
+      const uint32_t w = s_off[sl];
+      o = w >> 8;
+      o1 = o + (w & 0xffu);
+      b0 = __ldg(q.ent + o * 16u + lane);
+      if (PAL) c0 = __ldg(q.code + o * 16u + lane);
+      const int c = min(sl * 32 + lane, dimup - 1);
+      if (DOWN) {
+        eun = a.e_up[c];
+        mun = a.map_up[c];
+      } else {
+#pragma unroll
+        for (int r = 0; r < RT; ++r)
+          if (r < rows) hn[r] = ht[r * dimup + c];
+      }
+    }
+    while (sl < s1) {
+      const int iup = sl * 32 + lane;
+      const bool act = iup < dimup;
+      const int c = act ? iup : dimup - 1;  // inactive lanes work on a valid column, store nothing
+      const int nsl = sl + nw;
+      const bool more = nsl < s1;
+      const int cn = min(nsl * 32 + lane, dimup - 1);
+      uint32_t on = o, on1 = o1;
+      if (more) {
+        const uint32_t w = s_off[nsl];
+        on = w >> 8;
+        on1 = on + (w & 0xffu);
+      }
+      if (!DOWN) {
+        // The next tile's rows into L2 during the second half of this one: with one CTA per SM
+        // nothing else covers the staging, which took 9.3 us per 206 KB tile from HBM. Four
+        // 128-byte lines per slice; the first half's slices are fetched along with the second's.
+        const int64_t nr0 = r0 + int64_t(gridDim.x / q.csplit) * RT;
+        const int half = (s1 - s0) >> 1;
+        const int ps = lane < 4 ? sl : sl - half;
+        constexpr int kLine = 128 / int(sizeof(E));  // columns per line
+        const int pr = (lane & 3) / (32 / kLine), pc = ps * 32 + (lane & 3) % (32 / kLine) * kLine;
+        if (lane < 8 && sl - s0 >= half && nr0 + pr < a.dimdw && pc < dimup)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const E*>(a.v) + (nr0 + pr) * dimup + pc));
+      }
+      T up[RT];
+      if (LZ) {
+#pragma unroll
+        for (int r = 0; r < RT; ++r)
+          if (SUB && r < rows) up[r] = a.uprev[(r0 + r) * dimup + c];
+      }
+      T acc0[N];
+      if (DOWN) {
+        const ulonglong2 xc = S[c];
+        const T* xs = reinterpret_cast<const T*>(&xc);
+        const E* __restrict__ vc = reinterpret_cast<const E*>(a.v) + c;
+        const T eu = eun;
+        const uint32_t mu = mun;
+        eun = a.e_up[cn];
+        mun = a.map_up[cn];
+#pragma unroll
+        for (int r = 0; r < RT; ++r) {
+          if (r >= rows) {
+#pragma unroll
+            for (int w = 0; w < W; ++w) acc0[r * W + w] = T(0);
+            continue;
+          }
+          const T d0 = eu + s_edw[r] + a.U * T(__popc(mu & s_mdw[r]));
+          const T d = LZ ? T(double(d0) * sc) : d0;
+#pragma unroll
+          for (int w = 0; w < W; ++w) acc0[r * W + w] = d * xs[r * W + w];
+          const int n = s_cnt[r];
+          const H* lh = l_hop + r * q.cap;
+          int k = 0;
+          for (; k + KU <= n; k += KU) {  // KU independent source reads, then their terms in order
+            E x[KU];
+#pragma unroll
+            for (int u = 0; u < KU; ++u) x[u] = vc[lh[k + u].src];
+#pragma unroll
+            for (int u = 0; u < KU; ++u) elem_fma<T, W>(lh[k + u].val, x[u].x, acc0 + r * W);
+          }
+          if (k < n) {  // the rest: reads past the list repeat its last source
+            E x[KU];
+#pragma unroll
+            for (int u = 0; u < KU - 1; ++u) x[u] = vc[lh[min(k + u, n - 1)].src];
+#pragma unroll
+            for (int u = 0; u < KU - 1; ++u)
+              if (k + u < n) elem_fma<T, W>(lh[k + u].val, x[u].x, acc0 + r * W);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < RT; ++r)
+#pragma unroll
+          for (int w = 0; w < W; ++w) acc0[r * W + w] = hn[r].x[w];
+        if (more) {
+#pragma unroll
+          for (int r = 0; r < RT; ++r)
+            if (r < rows) hn[r] = ht[r * dimup + cn];
+        }
+      }
+      SlotAcc<T, W> acc;
+      acc.set(acc0);
+      for (uint32_t p = o; p < o1; p += 2) {
+        const uint4 wq = b0;
+        const uint2 cq = c0;
+        const uint32_t nx = (p + 2 < o1 ? p + 2 : on) * 16u + lane;
+        b0 = __ldg(q.ent + nx);
+        if (PAL) c0 = __ldg(q.code + nx);
+        const uint32_t ws[4] = {wq.x, wq.y, wq.z, wq.w};
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (u == 4 && p + 1 == o1) break;  // an odd number of half batches
+          const uint32_t ww = ws[u >> 1];
+          // bits 0..14 slot, bit 15 sign
+          const uint32_t at = sbase + ((u & 1) ? (ww >> 12) & 0x7fff0u : (ww << 4) & 0x7fff0u);
+          ulonglong2 x;
+          asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(x.x), "=l"(x.y) : "r"(at));
+          T h[W];
+          if (PAL) {
+            const T* pv = s_pal + (((u < 4 ? cq.x : cq.y) >> (8 * (u & 3))) & 0xffu) * W;
+#pragma unroll
+            for (int w = 0; w < W; ++w) h[w] = pv[w];
+          } else {
+            h[0] = flip_sign(hs, (u & 1) ? ww : ww << 16);
+          }
+          acc.fma(h, x);
+        }
+      }
+      if (LZ) {
+        // w = Hv - c * uprev; partial <v, w>
+        const double scl = s_lz[0], cc = s_lz[1];
+        const ulonglong2 xc = S[c];
+        const T* xs = reinterpret_cast<const T*>(&xc);
+#pragma unroll
+        for (int r = 0; r < RT; ++r)
+          if (act && r < rows) {
+            const T wt = SUB ? T(double(acc.get(r)) - cc * double(up[r])) : acc.get(r);
+            pa = __fma_rn(double(xs[r]) * scl, double(wt), pa);
+            T* p = a.hv + (r0 + r) * dimup + c;
+            if (DOWN) *p = wt;
+            else __stcs(p, wt);
+          }
+      } else {
+#pragma unroll
+        for (int r = 0; r < RT; ++r)
+          if (act && r < rows) {
+            E out;
+#pragma unroll
+            for (int w = 0; w < W; ++w) out.x[w] = acc.get(r * W + w);
+            if constexpr (W == 1) {
+              if (DOWN) ht[r * dimup + c] = out;
+              else __stcs(&ht[r * dimup + c].x[0], out.x[0]);
+            } else {
+              ht[r * dimup + c] = out;
+            }
+          }
+      }
+      sl = nsl;
+      o = on;
+      o1 = on1;
+    }
+    __syncthreads();
+  }
+  if (LZ) {  // block partial of <v, w>, fixed order
+    __shared__ double s_red[32];
+    for (int d = 16; d > 0; d >>= 1) pa += __shfl_down_sync(0xffffffffu, pa, d);
+    if (lane == 0) s_red[warp] = pa;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0.0;
+      for (int w = 0; w < nw; ++w) t += s_red[w];
+      a.partial[blockIdx.x] = t;
+    }
+    finish_in_last_block(a.partial, gridDim.x, a.red_out, 0);
+  }
+}
+
+template <typename T, int W, bool DOWN, bool LZ, bool PAL>
+int launch(const HxvArgs<T>& a, TileArgs<T, W>& q, cudaStream_t st, int sms) {
+  constexpr int RT = 16 / int(sizeof(T) * W);
+  const size_t smem = tile_smem(a.dimup, q.npal, RT * q.cap, sizeof(T) * W);
+  auto kern = k_tile<T, W, DOWN, LZ, PAL>;
+  if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  // 64 registers a thread: 1024 threads per SM, in as many CTAs as the tiles leave room for
+  const int per_sm = smem <= 54 * 1024 ? 4 : smem <= 111 * 1024 ? 2 : 1;
+  const int threads = 1024 / per_sm;
+  q.nsl = int((a.dimup + 31) / 32);
+  q.ntile = int((a.dimdw + RT - 1) / RT);
+  // whole product of a sector with few tiles: column parts of a tile, each staging the whole
+  // rows again, until three quarters of the resident CTAs have one (3x4 lattice, D = 853,776,
+  // one part against two: FP32, 231 tiles, 20.8 against 17.6 us; FP64, 462 tiles, 24.1 against
+  // 23.1, with four 26)
+  const int want = (3 * sms * per_sm / 4 + q.ntile - 1) / q.ntile;
+  const int most = std::max(1, q.nsl / (threads / 32));
+  q.csplit = DOWN ? std::max(1, std::min(want, most)) : 1;
+  int64_t g = int64_t(q.ntile) * q.csplit;
+  if (!DOWN || g > kRedMaxBlocks) g = std::min<int64_t>(g, DOWN ? kRedMaxBlocks : int64_t(sms) * per_sm);
+  kern<<<dim3(unsigned(g), a.ncols), threads, smem, st>>>(a, q);
+  EDG_CUDA(cudaGetLastError());
+  return EDG_OK;
+}
+
+template <typename T, int W, bool DOWN, bool LZ>
+int launch_pal(const HxvArgs<T>& a, TileArgs<T, W>& q, cudaStream_t st, int sms) {
+  if constexpr (W == 1) {
+    if (q.npal == 0) return launch<T, W, DOWN, LZ, false>(a, q, st, sms);
+  }
+  return launch<T, W, DOWN, LZ, true>(a, q, st, sms);
+}
+
+template <typename T, int W>
+int tile_pass(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, const T* vi_dw, bool down, bool lz,
+              cudaStream_t st, int sms) {
+  const int ord = sizeof(T) == 4 && W == 1 && up.t16_npal == 0 ? 1 : 0;  // FP32: the order-free schedule
+  TileArgs<T, W> q;
+  q.ent = reinterpret_cast<const uint4*>(up.t16_ent[ord].p);
+  q.code = reinterpret_cast<const uint2*>(up.t16_code.p);
+  q.off = up.t16_off[ord].p;
+  q.pal = up.t16_pal.p;
+  q.h = T(up.sell_h);
+  q.npal = up.t16_npal;
+  q.cap = down ? dw.max_row : 0;
+  q.vi_dw = vi_dw;
+  if constexpr (W == 1) {
+    if (lz) return down ? launch_pal<T, W, true, true>(a, q, st, sms) : launch_pal<T, W, false, true>(a, q, st, sms);
+  }
+  return down ? launch_pal<T, W, true, false>(a, q, st, sms) : launch_pal<T, W, false, false>(a, q, st, sms);
+}
+
+}  // namespace
+
+bool tile_available(const edg_sector_s* s, size_t elem, bool down) {
+  const SpinBasis& up = s->up;
+  if (!up.t16) return false;
+  const int rt = int(16 / elem);  // elem: bytes per vector element (a complex one counts whole)
+  return tile_smem(up.dim, up.t16_npal, down ? rt * s->dw.max_row : 0, elem) <= kTileSmemMax;
+}
+
+template <typename T>
+int tile_real(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, bool down, bool lz, cudaStream_t st,
+              int sms) {
+  return tile_pass<T, 1>(a, up, dw, nullptr, down, lz, st, sms);
+}
+template int tile_real<float>(const HxvArgs<float>&, const SpinBasis&, const SpinBasis&, bool, bool, cudaStream_t, int);
+template int tile_real<double>(const HxvArgs<double>&, const SpinBasis&, const SpinBasis&, bool, bool, cudaStream_t, int);
+
+
+template <typename T>
+int tile_cplx(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, const T* vi_dw, bool down,
+              cudaStream_t st, int sms) {
+  return tile_pass<T, 2>(a, up, dw, vi_dw, down, false, st, sms);
+}
+template int tile_cplx<float>(const HxvArgs<float>&, const SpinBasis&, const SpinBasis&, const float*, bool,
+                              cudaStream_t, int);
+template int tile_cplx<double>(const HxvArgs<double>&, const SpinBasis&, const SpinBasis&, const double*, bool,
+                               cudaStream_t, int);
+
+}  // namespace edg

@@ -501,7 +501,7 @@ int norm_dev(cudaStream_t st, const double* x, int64_t n, double* partial, doubl
 }
 
 int red_scratch_reset(cudaStream_t st, double* partial) {
-  EDG_CUDA(cudaMemsetAsync(partial + kRedBlocks, 0, sizeof(double), st));
+  EDG_CUDA(cudaMemsetAsync(partial + kRedMaxBlocks, 0, sizeof(double), st));
   return EDG_OK;
 }
 

@@ -129,14 +129,15 @@ int edg_hxv_d(edg_sector* s, int64_t nloc, const double* v, double* hv);
  * (nup = 4 for FP32, 1 for FP64): down 0 hop-balanced row groups, 1 block-staged rows (one
  * CTA per SM), 2 block-staged rows (two CTAs per SM), 3 the single-pass H x v (the whole
  * product in one launch, for vectors that sit in L2; the up choice is then unused); up (FP32)
- * 0 32-bit SELL schedule,
+ * 0 row tiles of 16-byte slots over a 16-bit schedule (rows of up to about 14,400 columns;
+ * 32-bit SELL schedule beyond),
  * 1 packed 16-bit schedule with negated copies, 2 packed 16-bit schedule with sign bits,
  * 3 Kronecker schedule (hops inside the low or the high half of the sites from per-half
  * tables, the rest from a per-column table). ms (may be NULL) receives each candidate's ms
  * per H x v, *ncand their number, *best the index kept. FP64 results are the same bits for
  * every pair; the FP32 packed and Kronecker up passes change the order of a row's terms.
- * Untuned real stored sectors of at most 500,000 states use the single pass (candidate 12
- * for FP32, 3 for FP64), other sectors candidate 0. No counterpart in the reference. */
+ * Untuned real stored sectors use the single pass (candidate 3 for FP64, 12 for FP32) up to
+ * 12,000,000 (FP64) and 4,000,000 (FP32) states, other sectors candidate 0. No counterpart in the reference. */
 int edg_sector_autotune(edg_sector* s, int precision, int reps, double* ms, int* ncand, int* best);
 /* Pin the H x v kernel pair of this sector for one precision to candidate k of
  * edg_sector_autotune's list (0..15 for FP32, 0..3 for FP64). The tables of the non-default
