@@ -21,7 +21,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
-#include <map>
 #include <mutex>
 #include <tuple>
 
@@ -251,11 +250,11 @@ __device__ __forceinline__ int between_parity(uint32_t t, int a, int b) {
   return __popc(t & mask) & 1;
 }
 
-// Row r of the stored hop table: sources ascending, value sign * Hij(a,b); with bhi (complex
-// Hij) also the imaginary parts, stored as -sign * Im Hij(a,b): the stored form keeps
-// conjg(Hij) (src/DIAG/stored/H_up.f90:19-21).
+// Row r of the hop table: sources ascending, value sign * Hij(a,b); with bhi (complex Hij) also
+// the imaginary parts, isign * sign * Im Hij(a,b): the stored form keeps conjg(Hij), isign = -1
+// (src/DIAG/stored/H_up.f90:19-21), the direct form applies Hij itself.
 __global__ void k_hop_fill(const uint32_t* map, int64_t dim, const int32_t* bonds, const double* bh,
-                           const double* bhi, int nb, const uint32_t* C, const uint32_t* off, uint32_t* src,
+                           const double* bhi, int nb, double isign, const uint32_t* C, const uint32_t* off, uint32_t* src,
                            double* v64, float* v32, double* v64i, float* v32i) {
   int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (r >= dim) return;
@@ -268,7 +267,7 @@ __global__ void k_hop_fill(const uint32_t* map, int64_t dim, const int32_t* bond
       uint32_t s = (t & ~(1u << a)) | (1u << b);
       const bool neg = between_parity(t, a, b);
       double v = neg ? -bh[k] : bh[k];
-      double vi = bhi ? (neg ? bhi[k] : -bhi[k]) : 0.0;
+      double vi = bhi ? (neg ? -isign : isign) * bhi[k] : 0.0;
       uint32_t j = rank_of(s, C);
       // insertion into the row, ascending source rank (the reference's summation order)
       uint32_t pos = n;
@@ -398,7 +397,8 @@ int build_tables(edg_sector_s* s, int spin, SpinBasis& B) {
     EDG_CHECK(B.val64i.alloc(nnz + 1, st, "hop values"));
     EDG_CHECK(B.val32i.alloc(nnz + 1, st, "hop values"));
   }
-  k_hop_fill<<<blocks, 256, 0, st>>>(B.map.p, B.dim, bonds.p, bh.p, s->cplx ? bhi.p : nullptr, nb, s->binom.p,
+  k_hop_fill<<<blocks, 256, 0, st>>>(B.map.p, B.dim, bonds.p, bh.p, s->cplx ? bhi.p : nullptr, nb,
+                                     s->form == EDG_FORM_STORED ? -1.0 : 1.0, s->binom.p,
                                      B.off.p, B.src.p, B.val64.p, B.val32.p, B.val64i.p, B.val32i.p);
   EDG_CUDA(cudaGetLastError());
   EDG_CUDA(cudaStreamSynchronize(st));
@@ -521,155 +521,195 @@ static void build_schedule(int64_t dim, int rt, const std::vector<uint32_t>& off
 // 16-bit slot schedule of the tile kernels (SpinBasis::t16_*): a 16-byte shared-memory load of a
 // warp is served 8 lanes at a time, and the 8 are served in one wavefront when their slots fall
 // in distinct 16-byte bank groups (slot % 8) or are the same slot. So each group of 8 columns of
-// a slice is scheduled on its own, and lanes with nothing to do in a slot read a zero slot of
-// a bank group that none of the 8 uses there.
-//  * ordered: each column's sources stay ascending; a lane whose next source clashes waits.
-//    Lanes with the most sources left go first. 23.3 slots for 17.1 hops on the 4x4
-//    half-filled sector (25.0 at the widest group of a slice), where unscheduled source order
-//    takes 39.1 wavefronts; XOR and multiplicative slot hashes and other groupings of the 32
-//    columns gave no fewer.
-//  * any order: an edge colouring of lanes x bank groups, 20.8 slots.
-// Entries are stored in batches of eight slots; a slice ends at a half batch.
-static bool schedule16(int64_t dim, bool ordered, const std::vector<uint32_t>& off, const std::vector<uint32_t>& src,
-                       const std::vector<uint8_t>& code, bool signs, std::vector<uint32_t>& soff,
-                       std::vector<uint16_t>& ent, std::vector<uint8_t>* codes) {
+// a slice is scheduled on its own, by one thread, and lanes with nothing to do in a slot read a
+// zero slot of a bank group that none of the 8 uses there. Lanes with the most sources left
+// go first.
+//  * ORDERED: each column's sources stay ascending; a lane whose next source clashes waits.
+//    23.3 slots for 17.1 hops on the 4x4 half-filled sector (25.0 at the widest group of a
+//    slice), where unscheduled source order takes 39.1 wavefronts; XOR and multiplicative slot
+//    hashes and other groupings of the 32 columns gave no fewer.
+//  * any order: each lane takes a source from the free bank group with the most sources left;
+//    20.85 slots (an optimal edge colouring: 20.81).
+// width != null: counts the slots of each group only. Otherwise fills the entries of a slice
+// that starts at batch soff >> 9 and has (soff & 511) half batches of four slots; entries are
+// stored in batches of eight slots.
+constexpr int kSchedMaxRow = 64;  // hops per column of the any-order schedule (a bit mask each)
+
+template <bool ORDERED>
+__global__ void k_sched16(int64_t dim, const uint32_t* __restrict__ off, const uint32_t* __restrict__ src,
+                          const uint8_t* __restrict__ code, bool signs, const uint32_t* __restrict__ soff,
+                          uint32_t* __restrict__ width, uint16_t* __restrict__ ent, uint8_t* __restrict__ codes) {
   constexpr int G = 8;
-  const int64_t nsl = (dim + 31) / 32;
-  soff.assign(nsl, 0);
-  ent.clear();
-  if (codes) codes->clear();
-  std::vector<std::pair<int, int>> edges;
-  std::vector<int> eidx, colour;
-  std::vector<int> slot;  // [slot][lane]: table index, -1 when idle
-  size_t nent = 0;
-  for (int64_t sl = 0; sl < nsl; ++sl) {
-    slot.clear();
-    size_t width = 1;
-    for (int g = 0; g < 32 / G; ++g) {
-      uint32_t pos[G], end[G];
-      size_t left = 0;
-      for (int l = 0; l < G; ++l) {
-        const int64_t r = sl * 32 + g * G + l;
-        pos[l] = r < dim ? off[r] : 0;
-        end[l] = r < dim ? off[r + 1] : 0;
-        left += end[l] - pos[l];
-      }
-      if (ordered) {
-        int ord[G];
-        for (int l = 0; l < G; ++l) ord[l] = l;
-        for (size_t c = 0; left; ++c) {
-          for (int i = 1; i < G; ++i)  // most sources left first (nearly sorted from slot to slot)
-            for (int j = i; j > 0 && end[ord[j]] - pos[ord[j]] > end[ord[j - 1]] - pos[ord[j - 1]]; --j)
-              std::swap(ord[j], ord[j - 1]);
-          int64_t used[G];
-          std::fill(used, used + G, int64_t(-1));
-          if (slot.size() < (c + 1) * 32) slot.resize((c + 1) * 32, -1);
-          for (int q = 0; q < G; ++q) {
-            const int l = ord[q];
-            if (pos[l] == end[l]) break;
-            const int64_t x = src[pos[l]];
-            if (used[x % G] < 0 || used[x % G] == x) {
-              used[x % G] = x;
-              slot[c * 32 + g * G + l] = int(pos[l]++);
-              --left;
-            }
-          }
-          width = std::max(width, c + 1);
-        }
-      } else {
-        edges.clear();
-        eidx.clear();
-        for (int l = 0; l < G; ++l)
-          for (uint32_t k = pos[l]; k < end[l]; ++k) {
-            edges.push_back({l, int(src[k] % G)});
-            eidx.push_back(int(k));
-          }
-        const int D = edge_colour(G, G, edges, colour);
-        if (D < 0) return false;
-        if (slot.size() < size_t(D) * 32) slot.resize(size_t(D) * 32, -1);
-        for (size_t i = 0; i < edges.size(); ++i) slot[size_t(colour[i]) * 32 + g * G + edges[i].first] = eidx[i];
-        width = std::max(width, size_t(D));
-      }
-    }
-    const size_t nb = (width + 7) / 8;
-    const uint32_t half = uint32_t((width + 3) / 4);
-    if (half > 255) return false;
-    soff[sl] = uint32_t(nent / 256) << 9 | half;
-    slot.resize(nb * 256, -1);
-    ent.resize(nent + nb * 256);
-    if (codes) codes->resize(nent + nb * 256, 0);
-    for (size_t c = 0; c < nb * 8; ++c)
-      for (int g = 0; g < 32 / G; ++g) {
-        const int* s = slot.data() + c * 32 + g * G;
-        unsigned used = 0;
-        for (int l = 0; l < G; ++l)
-          if (s[l] >= 0) used |= 1u << (src[s[l]] % G);
-        int fr = 0;
-        while (fr < G - 1 && ((used >> fr) & 1u)) ++fr;
-        const uint32_t zero = uint32_t(dim) + uint32_t((fr - int(dim % G) + G) % G);
-        for (int l = 0; l < G; ++l) {
-          const int k = s[l];
-          const size_t at = nent + (c / 8) * 256 + size_t(g * G + l) * 8 + c % 8;
-          ent[at] = uint16_t(k >= 0 ? src[k] | (signs ? uint32_t(code[k]) << 15 : 0u) : zero);
-          if (codes && k >= 0) (*codes)[at] = code[k];
-        }
-      }
-    nent += nb * 256;
+  const int64_t oct = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (oct >= (dim + 31) / 32 * 4) return;
+  uint32_t pos[G], left[G];
+  unsigned long long mask[G][G];  // any order: unused sources of a lane in a bank group
+  int ord[G], bank[G];
+  uint32_t total = 0;
+  for (int l = 0; l < G; ++l) {
+    const int64_t r = oct * G + l;
+    pos[l] = r < dim ? off[r] : 0;
+    left[l] = r < dim ? off[r + 1] - pos[l] : 0;
+    total += left[l];
+    ord[l] = l;
+    bank[l] = 0;
   }
-  return true;
+  if (!ORDERED) {
+    for (int l = 0; l < G; ++l)
+      for (int b = 0; b < G; ++b) mask[l][b] = 0;
+    for (int l = 0; l < G; ++l)
+      for (uint32_t k = 0; k < left[l]; ++k) {
+        const int b = int(src[pos[l] + k] % G);
+        mask[l][b] |= 1ull << k;
+        ++bank[b];
+      }
+  }
+  const uint32_t so = width ? 0u : soff[oct / 4];
+  const size_t base = size_t(so >> 9) * 256 + size_t(oct % 4) * G * 8;
+  const uint32_t slots = (so & 511u) * 4u;
+  for (uint32_t c = 0; total || (!width && c < (slots + 7) / 8 * 8); ++c) {
+    for (int i = 1; i < G; ++i)
+      for (int j = i; j > 0 && left[ord[j]] > left[ord[j - 1]]; --j) {
+        const int t = ord[j];
+        ord[j] = ord[j - 1];
+        ord[j - 1] = t;
+      }
+    uint32_t take[G], hold[G];  // the table index of each lane, the source held by each bank group
+    unsigned used = 0;
+    for (int l = 0; l < G; ++l) take[l] = 0xffffffffu;
+    for (int q = 0; q < G; ++q) {
+      const int l = ord[q];
+      if (left[l] == 0) break;
+      if (ORDERED) {
+        const uint32_t x = src[pos[l]];
+        const int b = int(x % G);
+        if (((used >> b) & 1u) && hold[b] != x) continue;
+        used |= 1u << b;
+        hold[b] = x;
+        take[l] = pos[l]++;
+      } else {
+        int best = -1;
+        for (int b = 0; b < G; ++b)
+          if (mask[l][b] && !((used >> b) & 1u) && (best < 0 || bank[b] > bank[best])) best = b;
+        if (best < 0) continue;
+        const int k = __ffsll(mask[l][best]) - 1;
+        mask[l][best] &= mask[l][best] - 1;
+        --bank[best];
+        used |= 1u << best;
+        take[l] = pos[l] + k;
+      }
+      --left[l];
+      --total;
+    }
+    if (width) {
+      width[oct] = c + 1;
+      continue;
+    }
+    int fr = 0;
+    while (fr < G - 1 && ((used >> fr) & 1u)) ++fr;
+    const uint32_t zero = uint32_t(dim) + uint32_t((fr - int(dim % G) + G) % G);
+    for (int l = 0; l < G; ++l) {
+      const size_t at = base + size_t(c / 8) * 256 + size_t(l) * 8 + c % 8;
+      const uint32_t k = take[l];
+      const bool on = k != 0xffffffffu;
+      ent[at] = uint16_t(on ? src[k] | (signs ? uint32_t(code[k]) << 15 : 0u) : zero);
+      if (codes) codes[at] = on ? code[k] : 0;
+    }
+  }
 }
 
-// Uploads the 16-bit schedules of one spin's hop table (val: values, vi: imaginary parts or
-// empty). Leaves B.t16 false where the tile kernels do not apply: rows whose slots exceed
-// shared memory, or more than 256 distinct values.
-int build_t16(edg_sector_s* s, SpinBasis& B, const std::vector<uint32_t>& off, const std::vector<uint32_t>& src,
-              const std::vector<double>& val, const std::vector<double>& vi) {
+// The code of every table value: its index in the palette of npal values (W doubles each).
+__global__ void k_code16(int64_t nnz, const double* __restrict__ val, const double* __restrict__ vi,
+                         const double* __restrict__ pal, int npal, uint8_t* __restrict__ code) {
+  const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (k >= nnz) return;
+  const int W = vi ? 2 : 1;
+  int c = 0;
+  while (c + 1 < npal && !(pal[c * W] == val[k] && (!vi || pal[c * W + 1] == vi[k]))) ++c;
+  code[k] = uint8_t(c);
+}
+
+// The 16-bit schedules of one spin's hop table, built on the device. Leaves B.t16 false where
+// the tile kernels do not apply: rows whose slots exceed shared memory, or more than 256
+// distinct values.
+int build_t16(edg_sector_s* s, const BondList& bl, SpinBasis& B) {
   cudaStream_t st = s->stream;
   B.t16 = false;
   B.t16_npal = 0;
   const int64_t dim = B.dim;
   if (dim < 1 || tile_smem(dim, 0, 0, 0) > kTileSmemMax) return EDG_OK;
-  std::vector<uint8_t> code(B.nnz + 1, 0);
+  const int W = s->cplx ? 2 : 1;
+  // the values a table can hold: each bond's with either sign (the stored form keeps conjg(Hij))
   std::vector<double> pal;
-  const bool uniform = vi.empty() && B.sell_uniform;
-  if (uniform) {
-    for (int64_t k = 0; k < B.nnz; ++k) code[k] = val[k] == B.sell_h ? 0 : 1;
+  if (!s->cplx && B.sell_uniform) {
+    pal = {B.sell_h, -B.sell_h};
   } else {
-    std::map<std::pair<double, double>, int> seen;
-    for (int64_t k = 0; k < B.nnz; ++k) {
-      const std::pair<double, double> v(val[k], vi.empty() ? 0.0 : vi[k]);
-      auto it = seen.find(v);
-      if (it == seen.end()) {
-        if (seen.size() == 256) return EDG_OK;
-        it = seen.emplace(v, int(seen.size())).first;
-        pal.push_back(v.first);
-        if (!vi.empty()) pal.push_back(v.second);
+    const double ci = s->form == EDG_FORM_STORED ? -1.0 : 1.0;
+    for (int k = 0; k < bl.nb; ++k)
+      for (double sg : {1.0, -1.0}) {
+        const double re = sg * bl.h[k], im = sg * ci * bl.hi[k];
+        bool seen = false;
+        for (size_t i = 0; i < pal.size() && !seen; i += W) seen = pal[i] == re && (W == 1 || pal[i + 1] == im);
+        if (seen) continue;
+        pal.push_back(re);
+        if (W == 2) pal.push_back(im);
       }
-      code[k] = uint8_t(it->second);
+    if (pal.empty()) pal.assign(W, 0.0);
+    const int npal = int(pal.size()) / W;
+    if (npal > 256 || tile_smem(dim, npal, 0, W * sizeof(double)) > kTileSmemMax) return EDG_OK;
+    B.t16_npal = npal;
+  }
+  const bool uniform = B.t16_npal == 0;
+  EDG_CHECK(B.t16_pal.alloc(pal.size(), st, "slot schedule"));
+  EDG_CUDA(cudaMemcpyAsync(B.t16_pal.p, pal.data(), pal.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+  DevBuf<uint8_t> code;
+  EDG_CHECK(code.alloc(B.nnz + 1, st, "slot schedule"));
+  if (B.nnz)
+    k_code16<<<unsigned((B.nnz + 255) / 256), 256, 0, st>>>(B.nnz, B.val64.p, s->cplx ? B.val64i.p : nullptr, B.t16_pal.p,
+                                                            int(pal.size()) / W, code.p);
+  const int64_t nsl = (dim + 31) / 32, noct = nsl * 4;
+  const unsigned grid = unsigned((noct + 31) / 32);
+  DevBuf<uint32_t> width;
+  EDG_CHECK(width.alloc(2 * noct, st, "slot schedule"));
+  const int norder = uniform ? 2 : 1;
+  EDG_CUDA(cudaMemsetAsync(width.p, 0, 2 * noct * sizeof(uint32_t), st));
+  const bool masks = B.max_row <= kSchedMaxRow;
+  for (int o = 0; o < norder; ++o) {
+    if (o == 0 || !masks)
+      k_sched16<true><<<grid, 32, 0, st>>>(dim, B.off.p, B.src.p, code.p, uniform, nullptr, width.p + o * noct, nullptr,
+                                           nullptr);
+    else
+      k_sched16<false><<<grid, 32, 0, st>>>(dim, B.off.p, B.src.p, code.p, uniform, nullptr, width.p + o * noct,
+                                            nullptr, nullptr);
+  }
+  EDG_CUDA(cudaGetLastError());
+  std::vector<uint32_t> w(2 * noct), soff(2 * nsl);
+  EDG_CUDA(cudaMemcpyAsync(w.data(), width.p, w.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  EDG_CUDA(cudaStreamSynchronize(st));
+  for (int o = 0; o < norder; ++o) {
+    uint32_t nb = 0;
+    for (int64_t sl = 0; sl < nsl; ++sl) {
+      uint32_t m = 1;
+      for (int g = 0; g < 4; ++g) m = std::max(m, w[o * noct + sl * 4 + g]);
+      const uint32_t half = (m + 3) / 4;
+      if (half > 511 || nb >= (1u << 23)) return EDG_OK;
+      soff[o * nsl + sl] = nb << 9 | half;
+      nb += (half + 1) / 2;
     }
-    if (seen.empty()) pal.assign(vi.empty() ? 1 : 2, 0.0);
-    B.t16_npal = int(std::max<size_t>(1, seen.size()));
-    if (tile_smem(dim, B.t16_npal, 0, vi.empty() ? 8 : 16) > kTileSmemMax) return EDG_OK;
+    EDG_CHECK(B.t16_off[o].alloc(nsl, st, "slot schedule"));
+    EDG_CHECK(B.t16_ent[o].alloc(size_t(nb) * 256, st, "slot schedule"));
+    if (!uniform) EDG_CHECK(B.t16_code.alloc(size_t(nb) * 256, st, "slot schedule"));
+    EDG_CUDA(cudaMemcpyAsync(B.t16_off[o].p, soff.data() + o * nsl, nsl * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+    uint8_t* codes = uniform ? nullptr : B.t16_code.p;
+    if (o == 0 || !masks)
+      k_sched16<true><<<grid, 32, 0, st>>>(dim, B.off.p, B.src.p, code.p, uniform, B.t16_off[o].p, nullptr,
+                                           B.t16_ent[o].p, codes);
+    else
+      k_sched16<false><<<grid, 32, 0, st>>>(dim, B.off.p, B.src.p, code.p, uniform, B.t16_off[o].p, nullptr,
+                                            B.t16_ent[o].p, codes);
   }
-  auto up = [&](void* d, const void* h, size_t bytes) { return cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, st); };
-  std::vector<uint32_t> soff;
-  std::vector<uint16_t> ent;
-  std::vector<uint8_t> codes;
-  for (int o = 0; o < (uniform ? 2 : 1); ++o) {
-    if (!schedule16(dim, o == 0, off, src, code, uniform, soff, ent, uniform ? nullptr : &codes)) return EDG_OK;
-    EDG_CHECK(B.t16_off[o].alloc(soff.size(), st, "slot schedule"));
-    EDG_CHECK(B.t16_ent[o].alloc(ent.size(), st, "slot schedule"));
-    EDG_CUDA(up(B.t16_off[o].p, soff.data(), soff.size() * sizeof(uint32_t)));
-    EDG_CUDA(up(B.t16_ent[o].p, ent.data(), ent.size() * sizeof(uint16_t)));
-    EDG_CUDA(cudaStreamSynchronize(st));  // the host vectors are reused
-  }
-  if (!uniform) {
-    EDG_CHECK(B.t16_code.alloc(codes.size(), st, "slot schedule"));
-    EDG_CHECK(B.t16_pal.alloc(pal.size(), st, "slot schedule"));
-    EDG_CUDA(up(B.t16_code.p, codes.data(), codes.size()));
-    EDG_CUDA(up(B.t16_pal.p, pal.data(), pal.size() * sizeof(double)));
-    EDG_CUDA(cudaStreamSynchronize(st));
-  }
+  EDG_CUDA(cudaGetLastError());
+  EDG_CUDA(cudaStreamSynchronize(st));  // host staging and the scratch go out of scope
   B.t16 = true;
   return EDG_OK;
 }
@@ -1058,19 +1098,14 @@ int build_variants(edg_sector_s* s, SpinBasis& B) {
 int build_sell(edg_sector_s* s, SpinBasis& B, bool up) {
   cudaStream_t st = s->stream;
   const int64_t dim = B.dim;
-  std::vector<uint32_t> off(dim + 1), src(B.nnz + 1);
-  std::vector<double> val(B.nnz + 1);
+  std::vector<uint32_t> off(dim + 1);
   EDG_CUDA(cudaMemcpyAsync(off.data(), B.off.p, (dim + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  if (B.nnz) {
-    EDG_CUDA(cudaMemcpyAsync(src.data(), B.src.p, B.nnz * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    EDG_CUDA(cudaMemcpyAsync(val.data(), B.val64.p, B.nnz * sizeof(double), cudaMemcpyDeviceToHost, st));
-  }
   EDG_CUDA(cudaStreamSynchronize(st));
   const int64_t nsl = (dim + 31) / 32;
   B.max_row = 0;
   for (int64_t r = 0; r < dim; ++r) B.max_row = std::max<int>(B.max_row, int(off[r + 1] - off[r]));
   // LPT grouping of rows for the down-spin pass: one group per resident CTA (4 per SM)
-  {
+  if (!up) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1107,22 +1142,22 @@ int build_sell(edg_sector_s* s, SpinBasis& B, bool up) {
     EDG_CUDA(cudaMemcpyAsync(B.group_rows.p, grows.data(), grows.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
     EDG_CUDA(cudaStreamSynchronize(st));
   }
-  double h0 = B.nnz ? std::fabs(val[0]) : 0.0;
-  bool uniform = true;
-  for (int64_t k = 0; k < B.nnz; ++k)
-    if (std::fabs(val[k]) != h0) { uniform = false; break; }
-  const double hsgn = B.nnz ? (val[0] < 0 ? -h0 : h0) : 0.0;  // value encoded by code 0
+  const BondList& bl = s->bonds[up ? 0 : 1];
+  const double hsgn = bl.nb ? bl.h[0] : 0.0;  // value encoded by code 0
+  bool uniform = !s->cplx;
+  for (int k = 0; k < bl.nb && uniform; ++k) uniform = std::fabs(bl.h[k]) == std::fabs(hsgn);
   B.sell_uniform = uniform;
   B.sell_h = hsgn;
   if (!up) return EDG_OK;
-  std::vector<double> vi;
-  if (s->cplx) {
-    vi.resize(B.nnz + 1);
-    if (B.nnz) EDG_CUDA(cudaMemcpyAsync(vi.data(), B.val64i.p, B.nnz * sizeof(double), cudaMemcpyDeviceToHost, st));
+  EDG_CHECK(build_t16(s, bl, B));
+  if (B.t16 || s->cplx || s->form != EDG_FORM_STORED) return EDG_OK;
+  std::vector<uint32_t> src(B.nnz + 1);
+  std::vector<double> val(B.nnz + 1);
+  if (B.nnz) {
+    EDG_CUDA(cudaMemcpyAsync(src.data(), B.src.p, B.nnz * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    EDG_CUDA(cudaMemcpyAsync(val.data(), B.val64.p, B.nnz * sizeof(double), cudaMemcpyDeviceToHost, st));
     EDG_CUDA(cudaStreamSynchronize(st));
   }
-  EDG_CHECK(build_t16(s, B, off, src, val, vi));
-  if (B.t16 || s->cplx) return EDG_OK;
   std::vector<uint32_t> soff(nsl + 1, 0);
   for (int64_t sl = 0; sl < nsl; ++sl) {
     uint32_t w = 0;

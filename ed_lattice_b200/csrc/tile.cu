@@ -3,7 +3,7 @@
 // A CTA stages the RT rows idw of a tile (4 FP32, 2 FP64, 2 complex64 or 1 complex128) column
 // by column: slot iup holds the RT values of column iup, so one 16-byte shared load per up hop
 // feeds RT rows. The up hops of 32 consecutive columns (a slice, one per lane) run slot by slot
-// over a 16-bit schedule (SpinBasis::t16_*, schedule16() in basis.cu). Two forms:
+// over a 16-bit schedule (SpinBasis::t16_*, k_sched16 in basis.cu). Two forms:
 //  * rows in (down == false): hv already holds diag*v and the down hops; hv += (I x H_up) v.
 //    The up pass of large sectors.
 //  * whole product (down == true): the diagonal, then the row's down hops (one list per row,
@@ -36,7 +36,7 @@ template <typename T, int W>
 struct TileArgs {
   const uint4* __restrict__ ent;       // eight 16-bit entries per lane and batch
   const uint2* __restrict__ code;      // eight palette codes per lane and batch (PAL)
-  const uint32_t* __restrict__ off;    // [nsl] first half batch (four slots) of a slice << 8 | half batches
+  const uint32_t* __restrict__ off;    // [nsl] first batch of a slice << 9 | its half batches (four slots)
   const double* __restrict__ pal;      // palette: W doubles per code (PAL)
   T h;                                 // value of sign bit 0 (!PAL)
   int npal = 0;
@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
     uint32_t mun = 0;
     if (sl < s1) {
       const uint32_t w = s_off[sl];
-      o = w >> 8;
-      o1 = o + (w & 0xffu);
+      o = (w >> 9) * 2;
+      o1 = o + (w & 511u);
       b0 = __ldg(q.ent + o * 16u + lane);
       if (PAL) c0 = __ldg(q.code + o * 16u + lane);
       const int c = min(sl * 32 + lane, dimup - 1);
@@ -229,8 +229,8 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
       uint32_t on = o, on1 = o1;
       if (more) {
         const uint32_t w = s_off[nsl];
-        on = w >> 8;
-        on1 = on + (w & 0xffu);
+        on = (w >> 9) * 2;
+        on1 = on + (w & 511u);
       }
       if (!DOWN) {
         // The next tile's rows into L2 during the second half of this one: with one CTA per SM
