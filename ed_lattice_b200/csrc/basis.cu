@@ -1294,11 +1294,10 @@ int sector_build(edg_sector_s* s) {
   s->dim = s->up.dim * s->dw.dim;
   s->vlen = s->cplx ? 2 * s->dim : s->dim;
   s->U = s->model.uloc;
-  if (s->form == EDG_FORM_STORED) {
-    EDG_CHECK(build_tables(s, 1, s->up));
-    EDG_CHECK(build_tables(s, 2, s->dw));
-  } else {
-    // direct form: bond lists only (both spins packed: [spin][k] -> a,b ; values)
+  EDG_CHECK(build_tables(s, 1, s->up));
+  EDG_CHECK(build_tables(s, 2, s->dw));
+  if (s->form != EDG_FORM_STORED) {
+    // direct form: also the bond lists (both spins packed: [spin][k] -> a,b ; values)
     std::vector<int32_t> hb;
     std::vector<double> hv, hvi;
     for (int sp = 0; sp < 2; ++sp) {

@@ -127,7 +127,7 @@ struct SpinBasis {
   DevBuf<double> e64;           // local one-body energy of each configuration [dim]
   DevBuf<float> e32;
   // Gather hop table over target rows: row r lists (source rank, value) with
-  // <r|H_sigma|src> = value, sources ascending. FORM_DIRECT keeps no table.
+  // <r|H_sigma|src> = value, sources ascending.
   DevBuf<uint32_t> off;         // [dim+1]
   DevBuf<uint32_t> src;         // [nnz]
   DevBuf<double> val64;         // [nnz]

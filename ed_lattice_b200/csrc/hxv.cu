@@ -1000,7 +1000,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_dw_blk(HxvArgs<T> a, const ui
 }
 
 // ---------------------------------------------------------------- direct (on-the-fly) form
-// No tables: each thread derives its hops from the bitstrings, as directMatVec does, with
+// For the sectors that the row tiles do not take. No tables: each thread derives its hops from the bitstrings, as directMatVec does, with
 // ranks from the combinatorial number system instead of binary_search. Bonds arrive
 // sorted by 2^b - 2^a so that sources come out in ascending rank.
 struct DirectArgsHdr {
@@ -1291,6 +1291,30 @@ int launch_up_smem(const HxvArgs<T>& a, const SellArgs<T>& sl, cudaStream_t st, 
   return EDG_OK;
 }
 
+// k_dw_grp over the row groups. FP32: 4 float2 segments per lane (256 columns per slab); FP64: 2
+// double2 segments, 4 hops in flight (3 in the Lanczos-scaled form, which spilled at 4 within
+// the 64 registers of 4 CTAs per SM).
+template <typename T, bool FIRST, bool SCALED>
+int launch_dw_grp(const HxvArgs<T>& a, const SpinBasis& Bdw, bool v2, cudaStream_t st) {
+  constexpr int NSEG = sizeof(T) == 4 ? 4 : 2;
+  constexpr int KU = sizeof(T) == 4 ? 3 : (SCALED ? 3 : 4);
+  auto kern = v2 ? k_dw_grp<T, 2, NSEG, KU, FIRST, SCALED> : k_dw_grp<T, 1, NSEG, KU, FIRST, SCALED>;
+  const int vec = v2 ? 2 : 1;
+  const size_t smem = size_t(Bdw.group_max) * (kDwHops * (sizeof(T) + 4) + sizeof(T) + 12) + 16;
+  if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  const int64_t nslab = (a.dimup + 32 * vec * NSEG - 1) / (32 * vec * NSEG);
+  kern<<<dim3(Bdw.groups, a.ncols), 256, smem, st>>>(a, Bdw.group_off.p, Bdw.group_rows.p, nslab, nullptr);
+  EDG_CUDA(cudaGetLastError());
+  return EDG_OK;
+}
+
+// hv += (H_dw x I) v by the row groups.
+template <typename T>
+int dw_add(const HxvArgs<T>& a, const SpinBasis& Bdw, cudaStream_t st) {
+  const bool v2 = a.dimup % 2 == 0 && reinterpret_cast<uintptr_t>(a.v) % (2 * sizeof(T)) == 0;
+  return launch_dw_grp<T, false, false>(a, Bdw, v2, st);
+}
+
 // VEC-wide loads need every row start aligned: DimUp a multiple of VEC and 2*sizeof(T)
 // aligned vector pointers (always true for our own buffers; checked for callers' pointers).
 // SCALED (Lanczos-fused mode) applies H to v = u / bn[jstep] by scaling the matrix elements.
@@ -1317,20 +1341,7 @@ int dw_pass(const HxvArgs<T>& a, const SpinBasis& Bdw, cudaStream_t st, int sms)
       return EDG_OK;
     }
   }
-  if (Bdw.max_row <= kDwHops && Bdw.groups > 0) {
-    // FP32: 4 float2 segments per lane (256 columns per slab); FP64: 2 double2 segments,
-    // 4 hops in flight (3 in the Lanczos-scaled form, which spilled at 4 within the 64
-    // registers of 4 CTAs per SM)
-    constexpr int NSEG = sizeof(T) == 4 ? 4 : 2;
-    constexpr int KU = sizeof(T) == 4 ? 3 : (SCALED ? 3 : 4);
-    auto kern = v2 ? k_dw_grp<T, 2, NSEG, KU, FIRST, SCALED> : k_dw_grp<T, 1, NSEG, KU, FIRST, SCALED>;
-    const size_t smem = size_t(Bdw.group_max) * (kDwHops * (sizeof(T) + 4) + sizeof(T) + 12) + 16;
-    if (smem > 48 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    const int64_t nslab = (a.dimup + 32 * vec * NSEG - 1) / (32 * vec * NSEG);
-    kern<<<dim3(Bdw.groups, a.ncols), 256, smem, st>>>(a, Bdw.group_off.p, Bdw.group_rows.p, nslab, nullptr);
-    EDG_CUDA(cudaGetLastError());
-    return EDG_OK;
-  }
+  if (Bdw.max_row <= kDwHops && Bdw.groups > 0) return launch_dw_grp<T, FIRST, SCALED>(a, Bdw, v2, st);
   if (SCALED || a.ncols > 1) {
     set_error("fused Lanczos and block H x V need the grouped down pass");
     return EDG_ERR_UNSUPPORTED;
@@ -1345,11 +1356,11 @@ int dw_pass(const HxvArgs<T>& a, const SpinBasis& Bdw, cudaStream_t st, int sms)
   return EDG_OK;
 }
 
-// diag*v and the down hops of a complex sector (k_dw_grp on complex elements).
-template <typename T>
+// The down hops of a complex sector (k_dw_grp on complex elements), after diag*v (FIRST) or added to hv.
+template <typename T, bool FIRST>
 int dw_pass_c(const HxvArgs<T>& a, const SpinBasis& Bdw, const T* vi_dw, cudaStream_t st) {
   constexpr int NSEG = sizeof(T) == 4 ? 4 : 2, KU = sizeof(T) == 4 ? 3 : 4;
-  auto kern = k_dw_grp<T, 2, NSEG, KU, true, false, 2>;
+  auto kern = k_dw_grp<T, 2, NSEG, KU, FIRST, false, 2>;
   const size_t smem = size_t(Bdw.group_max) * (kDwHops * (2 * sizeof(T) + 4) + sizeof(T) + 12) + 16;
   if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   const int64_t nslab = (a.dimup + 32 * NSEG - 1) / (32 * NSEG);
@@ -1439,7 +1450,7 @@ int up_pass(const HxvArgs<T>& a, edg_sector_s* s, cudaStream_t st, int sms, int*
     if (launch_up_kron<LZ>(a, B, st, sms, &status)) return status;
     if (launch_up_p16<LZ>(a, B, st, sms, &status)) return status;
   }
-  if (!FIRST && tile_available(s, sizeof(T), false)) return tile_real<T>(a, B, s->dw, false, LZ, st, sms);
+  if (!FIRST && tile_available(s, sizeof(T), false)) return tile_real<T>(a, B, s->dw, TileForm::kUpAdd, LZ, st, sms);
   const int rt = up_rows_per_cta(a.dimup, sizeof(T));
   if (rt == 0) {
     if (LZ || a.ncols > 1) {
@@ -1519,7 +1530,7 @@ HxvArgs<T> make_args(edg_sector_s* s, const T* v, T* hv) {
 template <typename T, bool LZ>
 int fused_pass(edg_sector_s* s, const HxvArgs<T>& a, cudaStream_t st, int sms) {
   if (tile_available(s, sizeof(T), true) && s->dim >= kTileMinDim)
-    return tile_real<T>(a, s->up, s->dw, true, LZ, st, sms);
+    return tile_real<T>(a, s->up, s->dw, TileForm::kDwUp, LZ, st, sms);
   const int64_t ntiles = a.dimdw * ((a.dimup + 31) / 32);
   const int64_t want = (ntiles + 7) / 8;
   int64_t g = want < int64_t(sms) * 8 ? want : int64_t(sms) * 8;
@@ -1541,17 +1552,22 @@ int hxv_apply(edg_sector_s* s, const T* v, T* hv) {
     const int64_t n = a.dimup * a.dimdw;
     const int64_t want = (n + 255) / 256;
     const int g = int(want < int64_t(sms) * 8 ? (want < 1 ? 1 : want) : int64_t(sms) * 8);
-    if (s->form == EDG_FORM_STORED) {
-      const T* vi = pick<T>(s->dw.val64i, s->dw.val32i);
-      // the tile kernels, in one launch while the source rows come from L2, else after the
-      // down pass over L2-sized column slabs
-      const bool vec = reinterpret_cast<uintptr_t>(v) % (2 * sizeof(T)) == 0 && reinterpret_cast<uintptr_t>(hv) % (2 * sizeof(T)) == 0;
-      if (vec && s->dim <= kFusedMaxDimC && tile_available(s, 2 * sizeof(T), true))
-        return tile_cplx<T>(a, s->up, s->dw, vi, true, st, sms);
-      if (vec && s->dw.max_row <= kDwHops && s->dw.groups > 0 && tile_available(s, 2 * sizeof(T), false)) {
-        EDG_CHECK(dw_pass_c<T>(a, s->dw, vi, st));
-        return tile_cplx<T>(a, s->up, s->dw, nullptr, false, st, sms);
+    // the tile kernels, in one launch while the source rows come from L2, else with the down
+    // pass over L2-sized column slabs
+    const bool stored = s->form == EDG_FORM_STORED;
+    const T* vi = pick<T>(s->dw.val64i, s->dw.val32i);
+    const bool vec = reinterpret_cast<uintptr_t>(v) % (2 * sizeof(T)) == 0 && reinterpret_cast<uintptr_t>(hv) % (2 * sizeof(T)) == 0;
+    if (vec && s->dim <= kFusedMaxDimC && tile_available(s, 2 * sizeof(T), true))
+      return tile_cplx<T>(a, s->up, s->dw, vi, stored ? TileForm::kDwUp : TileForm::kUpDw, st, sms);
+    if (vec && s->dw.max_row <= kDwHops && s->dw.groups > 0 && tile_available(s, 2 * sizeof(T), false)) {
+      if (stored) {
+        EDG_CHECK((dw_pass_c<T, true>(a, s->dw, vi, st)));
+        return tile_cplx<T>(a, s->up, s->dw, nullptr, TileForm::kUpAdd, st, sms);
       }
+      EDG_CHECK((tile_cplx<T>(a, s->up, s->dw, nullptr, TileForm::kUp, st, sms)));
+      return dw_pass_c<T, false>(a, s->dw, vi, st);
+    }
+    if (stored) {
       k_cplx_stored<T><<<g, 256, 0, st>>>(a, pick<T>(s->up.val64i, s->up.val32i), pick<T>(s->dw.val64i, s->dw.val32i));
     } else {
       DirectArgsHdr d;
@@ -1574,6 +1590,14 @@ int hxv_apply(edg_sector_s* s, const T* v, T* hv) {
     EDG_CHECK((dw_pass<T, true, false>(a, s->dw, st, sms)));
     EDG_CHECK((up_pass<T, false, false>(a, s, st, sms, nullptr)));
   } else {
+    // By row tiles (4x4 (6,6), FP64 / FP32: 1.44 / 0.61 ms, against 6.44 / 5.62 by k_direct_rows,
+    // whose up gathers scatter over global memory; 3x4 (6,6) 25 / 19 us against 126 / 119). The bitstring kernels serve the rows and hop lists that those do not take.
+    if (s->dim <= (sizeof(T) == 8 ? kFusedMaxDim64 : kFusedMaxDim32) && tile_available(s, sizeof(T), true))
+      return tile_real<T>(a, s->up, s->dw, TileForm::kUpDw, false, st, sms);
+    if (s->dw.max_row <= kDwHops && s->dw.groups > 0 && tile_available(s, sizeof(T), false)) {
+      EDG_CHECK((tile_real<T>(a, s->up, s->dw, TileForm::kUp, false, st, sms)));
+      return dw_add<T>(a, s->dw, st);
+    }
     DirectArgsHdr d;
     d.nb_up = s->bonds[0].nb;
     d.nb_dw = s->bonds[1].nb;

@@ -124,14 +124,15 @@ __device__ __forceinline__ double flip_sign(double h, uint32_t e) {
   return __longlong_as_double(__double_as_longlong(h) ^ (static_cast<long long>(e & 0x80000000u) << 32));
 }
 
-// ---- tile.cu: (diag + H_dw) v (down) and (I x H_up) v of a real stored sector, plain or as
-// the Lanczos-fused step (lz), over the rows of `a` (see tile.cu)
+// ---- tile.cu: the parts of H x v that a row-tile launch computes (see there), for the rows of
+// `a`, plain or (lz: kUpAdd and kDwUp) as the Lanczos-fused step
+enum class TileForm { kUpAdd, kDwUp, kUpDw, kUp };
 template <typename T>
-int tile_real(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, bool down, bool lz, cudaStream_t st,
+int tile_real(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, TileForm form, bool lz, cudaStream_t st,
               int sms);
-// The same for a complex stored sector (vi_dw: imaginary parts of the down values).
+// The same for a complex sector (vi_dw: imaginary parts of the down values).
 template <typename T>
-int tile_cplx(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, const T* vi_dw, bool down,
+int tile_cplx(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, const T* vi_dw, TileForm form,
               cudaStream_t st, int sms);
 
 }  // namespace edg

@@ -3,15 +3,17 @@
 // A CTA stages the RT rows idw of a tile (4 FP32, 2 FP64, 2 complex64 or 1 complex128) column
 // by column: slot iup holds the RT values of column iup, so one 16-byte shared load per up hop
 // feeds RT rows. The up hops of 32 consecutive columns (a slice, one per lane) run slot by slot
-// over a 16-bit schedule (SpinBasis::t16_*, k_sched16 in basis.cu). Two forms:
-//  * rows in (down == false): hv already holds diag*v and the down hops; hv += (I x H_up) v.
-//    The up pass of large sectors.
-//  * whole product (down == true): the diagonal, then the row's down hops (one list per row,
-//    the same for every lane: coalesced reads of the source rows), then the up hops. One launch
-//    and one write of hv; the source rows come from L2, so it is the H x v of sectors whose
-//    vectors sit there.
-// Both add the terms of an element in the stored form's order (diag, DW, UP; sources
-// ascending), so FP64 results carry the same bits as spMatVec's restatement.
+// over a 16-bit schedule (SpinBasis::t16_*, k_sched16 in basis.cu). Forms:
+//  * kUpAdd: hv already holds diag*v and the down hops; hv += (I x H_up) v. The up pass of
+//    large stored sectors.
+//  * kDwUp: the whole product, the diagonal, then the row's down hops (one list per row, the
+//    same for every lane: coalesced reads of the source rows), then the up hops. One launch and
+//    one write of hv; the source rows come from L2, so it is the H x v of sectors whose vectors
+//    sit there.
+//  * kUpDw, kUp: the direct form's order, diag, UP, DW: whole, or without the down hops, which
+//    the down pass then adds.
+// Sources come ascending inside each spin part, so FP64 results carry the bits of spMatVec's
+// and directMatVec's restatements.
 //
 // What bounds it: the shared-memory data path, 128 bytes per clock and SM. A slot of a slice
 // takes 4 wavefronts (one per 8 lanes) and half a wavefront of entries; in source order without
@@ -121,12 +123,14 @@ struct alignas(8) Hop {
   uint32_t src;
 };
 
-template <typename T, int W, bool DOWN, bool LZ, bool PAL>
+template <typename T, int W, TileForm FORM, bool LZ, bool PAL>
 __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q) {
   if (!select_column(a)) return;
   constexpr int RT = 16 / int(sizeof(T) * W);  // rows per tile
   constexpr int N = RT * W;                    // reals per slot
   constexpr int KU = 8 / W;                    // down hops in flight
+  constexpr bool DIAG = FORM != TileForm::kUpAdd;                            // starts from diag*v, not hv
+  constexpr bool DOWN = FORM == TileForm::kDwUp || FORM == TileForm::kUpDw;  // down hops here
   // uprev is subtracted here, after all hops, unless the down pass began from -c * uprev
   constexpr bool SUB = LZ && (DOWN || !lz_sub_in_dw<T>());
   using E = Elem<T, W>;
@@ -174,12 +178,12 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
         if (r < rows) xs[r] = vt[r * dimup + j];
       S[j] = slot;
     }
-    if (DOWN) {
+    if (DIAG) {
 #pragma unroll
       for (int r = 0; r < RT; ++r) {
         if (r >= rows) break;
         const uint32_t k0 = a.off_dw[r0 + r], n = a.off_dw[r0 + r + 1] - k0;
-        for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
+        for (uint32_t k = threadIdx.x; DOWN && k < n; k += blockDim.x) {
           H h;
           h.val[0] = LZ ? T(double(a.val_dw[k0 + k]) * sc) : a.val_dw[k0 + k];
           if (W == 2) h.val[W - 1] = q.vi_dw[k0 + k];
@@ -210,7 +214,7 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
       b0 = __ldg(q.ent + o * 16u + lane);
       if (PAL) c0 = __ldg(q.code + o * 16u + lane);
       const int c = min(sl * 32 + lane, dimup - 1);
-      if (DOWN) {
+      if (DIAG) {
         eun = a.e_up[c];
         mun = a.map_up[c];
       } else {
@@ -250,11 +254,36 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
         for (int r = 0; r < RT; ++r)
           if (SUB && r < rows) up[r] = a.uprev[(r0 + r) * dimup + c];
       }
+      // acc += the down hops of the tile's rows
+      auto down_hops = [&](T* acc) {
+        const E* __restrict__ vc = reinterpret_cast<const E*>(a.v) + c;
+#pragma unroll
+        for (int r = 0; r < RT; ++r) {
+          if (r >= rows) break;
+          const int n = s_cnt[r];
+          const H* lh = l_hop + r * q.cap;
+          int k = 0;
+          for (; k + KU <= n; k += KU) {  // KU independent source reads, then their terms in order
+            E x[KU];
+#pragma unroll
+            for (int u = 0; u < KU; ++u) x[u] = vc[lh[k + u].src];
+#pragma unroll
+            for (int u = 0; u < KU; ++u) elem_fma<T, W>(lh[k + u].val, x[u].x, acc + r * W);
+          }
+          if (k < n) {  // the rest: reads past the list repeat its last source
+            E x[KU];
+#pragma unroll
+            for (int u = 0; u < KU - 1; ++u) x[u] = vc[lh[min(k + u, n - 1)].src];
+#pragma unroll
+            for (int u = 0; u < KU - 1; ++u)
+              if (k + u < n) elem_fma<T, W>(lh[k + u].val, x[u].x, acc + r * W);
+          }
+        }
+      };
       T acc0[N];
-      if (DOWN) {
+      if (DIAG) {
         const ulonglong2 xc = S[c];
         const T* xs = reinterpret_cast<const T*>(&xc);
-        const E* __restrict__ vc = reinterpret_cast<const E*>(a.v) + c;
         const T eu = eun;
         const uint32_t mu = mun;
         eun = a.e_up[cn];
@@ -270,25 +299,8 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
           const T d = LZ ? T(double(d0) * sc) : d0;
 #pragma unroll
           for (int w = 0; w < W; ++w) acc0[r * W + w] = d * xs[r * W + w];
-          const int n = s_cnt[r];
-          const H* lh = l_hop + r * q.cap;
-          int k = 0;
-          for (; k + KU <= n; k += KU) {  // KU independent source reads, then their terms in order
-            E x[KU];
-#pragma unroll
-            for (int u = 0; u < KU; ++u) x[u] = vc[lh[k + u].src];
-#pragma unroll
-            for (int u = 0; u < KU; ++u) elem_fma<T, W>(lh[k + u].val, x[u].x, acc0 + r * W);
-          }
-          if (k < n) {  // the rest: reads past the list repeat its last source
-            E x[KU];
-#pragma unroll
-            for (int u = 0; u < KU - 1; ++u) x[u] = vc[lh[min(k + u, n - 1)].src];
-#pragma unroll
-            for (int u = 0; u < KU - 1; ++u)
-              if (k + u < n) elem_fma<T, W>(lh[k + u].val, x[u].x, acc0 + r * W);
-          }
         }
+        if (FORM == TileForm::kDwUp) down_hops(acc0);
       } else {
 #pragma unroll
         for (int r = 0; r < RT; ++r)
@@ -328,6 +340,10 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
           acc.fma(h, x);
         }
       }
+      T res[N];
+#pragma unroll
+      for (int i = 0; i < N; ++i) res[i] = acc.get(i);
+      if (FORM == TileForm::kUpDw) down_hops(res);
       if (LZ) {
         // w = Hv - c * uprev; partial <v, w>
         const double scl = s_lz[0], cc = s_lz[1];
@@ -336,7 +352,7 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
 #pragma unroll
         for (int r = 0; r < RT; ++r)
           if (act && r < rows) {
-            const T wt = SUB ? T(double(acc.get(r)) - cc * double(up[r])) : acc.get(r);
+            const T wt = SUB ? T(double(res[r]) - cc * double(up[r])) : res[r];
             pa = __fma_rn(double(xs[r]) * scl, double(wt), pa);
             T* p = a.hv + (r0 + r) * dimup + c;
             if (DOWN) *p = wt;
@@ -348,7 +364,7 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
           if (act && r < rows) {
             E out;
 #pragma unroll
-            for (int w = 0; w < W; ++w) out.x[w] = acc.get(r * W + w);
+            for (int w = 0; w < W; ++w) out.x[w] = res[r * W + w];
             if constexpr (W == 1) {
               if (DOWN) ht[r * dimup + c] = out;
               else __stcs(&ht[r * dimup + c].x[0], out.x[0]);
@@ -377,11 +393,12 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
   }
 }
 
-template <typename T, int W, bool DOWN, bool LZ, bool PAL>
+template <typename T, int W, TileForm FORM, bool LZ, bool PAL>
 int launch(const HxvArgs<T>& a, TileArgs<T, W>& q, cudaStream_t st, int sms) {
   constexpr int RT = 16 / int(sizeof(T) * W);
+  constexpr bool DOWN = FORM == TileForm::kDwUp || FORM == TileForm::kUpDw;
   const size_t smem = tile_smem(a.dimup, q.npal, RT * q.cap, sizeof(T) * W);
-  auto kern = k_tile<T, W, DOWN, LZ, PAL>;
+  auto kern = k_tile<T, W, FORM, LZ, PAL>;
   if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   // 64 registers a thread: 1024 threads per SM, in as many CTAs as the tiles leave room for
   const int per_sm = smem <= 54 * 1024 ? 4 : smem <= 111 * 1024 ? 2 : 1;
@@ -402,16 +419,16 @@ int launch(const HxvArgs<T>& a, TileArgs<T, W>& q, cudaStream_t st, int sms) {
   return EDG_OK;
 }
 
-template <typename T, int W, bool DOWN, bool LZ>
+template <typename T, int W, TileForm FORM, bool LZ>
 int launch_pal(const HxvArgs<T>& a, TileArgs<T, W>& q, cudaStream_t st, int sms) {
   if constexpr (W == 1) {
-    if (q.npal == 0) return launch<T, W, DOWN, LZ, false>(a, q, st, sms);
+    if (q.npal == 0) return launch<T, W, FORM, LZ, false>(a, q, st, sms);
   }
-  return launch<T, W, DOWN, LZ, true>(a, q, st, sms);
+  return launch<T, W, FORM, LZ, true>(a, q, st, sms);
 }
 
 template <typename T, int W>
-int tile_pass(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, const T* vi_dw, bool down, bool lz,
+int tile_pass(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, const T* vi_dw, TileForm form, bool lz,
               cudaStream_t st, int sms) {
   const int ord = sizeof(T) == 4 && W == 1 && up.t16_npal == 0 ? 1 : 0;  // FP32: the order-free schedule
   TileArgs<T, W> q;
@@ -421,12 +438,19 @@ int tile_pass(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, con
   q.pal = up.t16_pal.p;
   q.h = T(up.sell_h);
   q.npal = up.t16_npal;
-  q.cap = down ? dw.max_row : 0;
+  q.cap = form == TileForm::kDwUp || form == TileForm::kUpDw ? dw.max_row : 0;
   q.vi_dw = vi_dw;
   if constexpr (W == 1) {
-    if (lz) return down ? launch_pal<T, W, true, true>(a, q, st, sms) : launch_pal<T, W, false, true>(a, q, st, sms);
+    if (lz)
+      return form == TileForm::kDwUp ? launch_pal<T, W, TileForm::kDwUp, true>(a, q, st, sms)
+                                     : launch_pal<T, W, TileForm::kUpAdd, true>(a, q, st, sms);
   }
-  return down ? launch_pal<T, W, true, false>(a, q, st, sms) : launch_pal<T, W, false, false>(a, q, st, sms);
+  switch (form) {
+    case TileForm::kUpAdd: return launch_pal<T, W, TileForm::kUpAdd, false>(a, q, st, sms);
+    case TileForm::kDwUp: return launch_pal<T, W, TileForm::kDwUp, false>(a, q, st, sms);
+    case TileForm::kUpDw: return launch_pal<T, W, TileForm::kUpDw, false>(a, q, st, sms);
+    default: return launch_pal<T, W, TileForm::kUp, false>(a, q, st, sms);
+  }
 }
 
 }  // namespace
@@ -439,22 +463,23 @@ bool tile_available(const edg_sector_s* s, size_t elem, bool down) {
 }
 
 template <typename T>
-int tile_real(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, bool down, bool lz, cudaStream_t st,
+int tile_real(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, TileForm form, bool lz, cudaStream_t st,
               int sms) {
-  return tile_pass<T, 1>(a, up, dw, nullptr, down, lz, st, sms);
+  return tile_pass<T, 1>(a, up, dw, nullptr, form, lz, st, sms);
 }
-template int tile_real<float>(const HxvArgs<float>&, const SpinBasis&, const SpinBasis&, bool, bool, cudaStream_t, int);
-template int tile_real<double>(const HxvArgs<double>&, const SpinBasis&, const SpinBasis&, bool, bool, cudaStream_t, int);
-
+template int tile_real<float>(const HxvArgs<float>&, const SpinBasis&, const SpinBasis&, TileForm, bool, cudaStream_t,
+                              int);
+template int tile_real<double>(const HxvArgs<double>&, const SpinBasis&, const SpinBasis&, TileForm, bool, cudaStream_t,
+                               int);
 
 template <typename T>
-int tile_cplx(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, const T* vi_dw, bool down,
+int tile_cplx(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, const T* vi_dw, TileForm form,
               cudaStream_t st, int sms) {
-  return tile_pass<T, 2>(a, up, dw, vi_dw, down, false, st, sms);
+  return tile_pass<T, 2>(a, up, dw, vi_dw, form, false, st, sms);
 }
-template int tile_cplx<float>(const HxvArgs<float>&, const SpinBasis&, const SpinBasis&, const float*, bool,
+template int tile_cplx<float>(const HxvArgs<float>&, const SpinBasis&, const SpinBasis&, const float*, TileForm,
                               cudaStream_t, int);
-template int tile_cplx<double>(const HxvArgs<double>&, const SpinBasis&, const SpinBasis&, const double*, bool,
+template int tile_cplx<double>(const HxvArgs<double>&, const SpinBasis&, const SpinBasis&, const double*, TileForm,
                                cudaStream_t, int);
 
 }  // namespace edg

@@ -40,7 +40,10 @@ enum {
 
 /* H x v forms: the reference's ed_sparse_H switch (src/INPUT_VARS.f90:151,
  * src/DIAG/HAMILTONIAN.f90:148-160). STORED = spMatVec over tables built once per sector;
- * DIRECT = directMatVec, matrix elements generated on the fly. */
+ * DIRECT = directMatVec: its summation order (diagonal, up, down), its use of Hij without
+ * conjugation and its ed_filling rule for the diagonal. The tables of one spin take O(DimUp) or
+ * O(DimDw) bytes, so both forms run from them; matrix elements are generated on the fly only
+ * for rows beyond shared memory or more than 32 hops per row. */
 enum { EDG_FORM_STORED = 0, EDG_FORM_DIRECT = 1 };
 
 /* Precision of the device Lanczos vectors. Scalars (alpha, beta, dots) are always FP64. */

@@ -81,6 +81,28 @@ def test_hxv_tile_vs_oracle(case):
     s.delete()
 
 
+@pytest.mark.parametrize("case", CASES + [(4, 4, 5, 4, 0.0)], ids=lambda c: "%dx%d_%d_%d_%g" % c)
+def test_hxv_tile_direct(case):
+    """The direct form's order (diag, UP, DW), whole (up to 12,000,000 FP64 and 4,000,000 FP32
+    states) and, last case in FP32, as two passes."""
+    import torch
+    lx, ly, nup, ndw, tp = case
+    h = lattice(lx, ly, tp)
+    s = E.Sector(E.Model(h, uloc=4.0, xmu=2.0, hfmode=False), nup, ndw, E.EDG_FORM_DIRECT)
+    s.set_stream(torch.cuda.current_stream().cuda_stream)
+    v = O.random_vector(3, s.dim)
+    ref = O.direct_matvec_d(O.Model(h, uloc=4.0, xmu=2.0, hfmode=False), nup, ndw, v)
+    x = torch.from_numpy(v).cuda()
+    y = torch.full_like(x, float("nan"))
+    L.check(L.lib().edg_hxv_dev_f64(s.handle, C.c_void_p(x.data_ptr()), C.c_void_p(y.data_ptr())), "hxv")
+    assert np.array_equal(y.cpu().numpy(), ref)
+    x = x.float()
+    y = torch.full_like(x, float("nan"))
+    L.check(L.lib().edg_hxv_dev_f32(s.handle, C.c_void_p(x.data_ptr()), C.c_void_p(y.data_ptr())), "hxv")
+    assert np.abs(y.cpu().numpy() - ref).max() <= 2e-6 * np.abs(ref).max()
+    s.delete()
+
+
 def test_infinities_stay_where_they_belong():
     """An infinite element of v reaches only the rows that H connects to it: idle slots and the
     repeated reads of short hop lists add nothing."""
@@ -115,16 +137,18 @@ def flux_lattice(lx, ly, flux):
 @pytest.mark.parametrize("case", [(8, 1, 0, 4), (8, 1, 4, 0), (3, 3, 4, 5), (11, 1, 5, 4), (3, 4, 6, 5), (7, 2, 7, 3),
                                   (5, 3, 7, 2), (4, 4, 8, 1), (4, 4, 5, 5)], ids=lambda c: "%dx%d_%d_%d" % c)
 @pytest.mark.parametrize("prec", ["f64", "f32"])
-def test_hxv_tile_complex(case, prec):
+@pytest.mark.parametrize("form", [E.EDG_FORM_STORED, E.EDG_FORM_DIRECT], ids=["stored", "direct"])
+def test_hxv_tile_complex(case, prec, form):
     """Complex Hij: one launch up to 10,000,000 states, down pass and row tiles beyond (the last
     case). FP64 to 1e-13 of the largest element, FP32 to 2e-6."""
     import torch
     lx, ly, nup, ndw = case
     h = flux_lattice(lx, ly, 0.25)
-    s = E.Sector(E.Model(h, uloc=4.0, xmu=2.0, hfmode=False), nup, ndw)
+    s = E.Sector(E.Model(h, uloc=4.0, xmu=2.0, hfmode=False), nup, ndw, form)
     s.set_stream(torch.cuda.current_stream().cuda_stream)
     v = O.random_vector(3, s.dim) + 1j * O.random_vector(4, s.dim)
-    ref = O.Stored(O.Model(h, uloc=4.0, xmu=2.0, hfmode=False), nup, ndw).matvec_z(v)
+    om = O.Model(h, uloc=4.0, xmu=2.0, hfmode=False)
+    ref = O.Stored(om, nup, ndw).matvec_z(v) if form == E.EDG_FORM_STORED else O.direct_matvec_z(om, nup, ndw, v)
     x = torch.from_numpy(v).cuda().to(torch.complex128 if prec == "f64" else torch.complex64)
     y = torch.full_like(x, float("nan"))
     fn = L.lib().edg_hxv_dev_f64 if prec == "f64" else L.lib().edg_hxv_dev_f32
