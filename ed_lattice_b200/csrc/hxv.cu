@@ -570,6 +570,56 @@ struct VecLd<double, 2> {
   }
 };
 
+template <typename T, int VEC>
+struct VecSt;  // VEC-wide streaming store
+template <typename T>
+struct VecSt<T, 1> {
+  static __device__ __forceinline__ void store(T* p, const T* x) { __stcs(p, x[0]); }
+};
+template <>
+struct VecSt<float, 2> {
+  static __device__ __forceinline__ void store(float* p, const float* x) {
+    __stcs(reinterpret_cast<float2*>(p), make_float2(x[0], x[1]));
+  }
+};
+template <>
+struct VecSt<double, 2> {
+  static __device__ __forceinline__ void store(double* p, const double* x) {
+    __stcs(reinterpret_cast<double2*>(p), make_double2(x[0], x[1]));
+  }
+};
+template <typename T, int VEC>
+struct VecLds {  // VEC-wide shared-memory load
+  static __device__ __forceinline__ void load(const T* p, T* x) {
+#pragma unroll
+    for (int r = 0; r < VEC; ++r) x[r] = p[r];
+  }
+};
+template <>
+struct VecLds<float, 2> {
+  static __device__ __forceinline__ void load(const float* p, float* x) {
+    const float2 t = *reinterpret_cast<const float2*>(p);
+    x[0] = t.x;
+    x[1] = t.y;
+  }
+};
+template <>
+struct VecLds<uint32_t, 2> {
+  static __device__ __forceinline__ void load(const uint32_t* p, uint32_t* x) {
+    const uint2 t = *reinterpret_cast<const uint2*>(p);
+    x[0] = t.x;
+    x[1] = t.y;
+  }
+};
+template <>
+struct VecLds<double, 2> {
+  static __device__ __forceinline__ void load(const double* p, double* x) {
+    const double2 t = *reinterpret_cast<const double2*>(p);
+    x[0] = t.x;
+    x[1] = t.y;
+  }
+};
+
 template <typename T, int VEC, bool FIRST>
 __global__ void __launch_bounds__(256) k_dw_seg(HxvArgs<T> a, int64_t ntiles) {
   const int lane = threadIdx.x & 31;
@@ -721,7 +771,7 @@ __global__ void __launch_bounds__(256) k_hxv_fused(HxvArgs<T> a, int64_t ntiles)
 // is read once per hop; no global load of the hop list sits in the inner loop.
 constexpr int kDwHops = 32;  // hop-list capacity per row held in shared memory
 
-template <typename T, int VEC, int NSEG, int KU, bool FIRST, bool SCALED, int W = 1>
+template <typename T, int VEC, int NSEG, int KU, int PARTS, bool FIRST, bool SCALED, int W = 1>
 __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t* __restrict__ goff,
                                                 const uint32_t* __restrict__ grows, int64_t nslab,
                                                 const T* __restrict__ vi_dw = nullptr) {
@@ -767,18 +817,52 @@ __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t*
   static_assert(W == 1 || VEC == 2, "a lane reads one complex element");
   constexpr int EPL = VEC / W;    // elements per lane
   constexpr int SEGW = 32 * EPL;  // columns per warp-wide segment
+  constexpr int PARTW = SEGW * NSEG;
+  constexpr int SLABW = PARTW * PARTS;  // columns between two barriers
+  // The slab's column terms of the diagonal, read by every row: from global memory they were two
+  // loads per element next to the 17 of the hops (4x4 (6,6) FP32: 359 us with them there). The
+  // next slab's are loaded while this one runs.
+  constexpr int CPT = (SLABW + 255) / 256;  // columns per thread
+  __shared__ __align__(16) T s_eup[SLABW];
+  __shared__ __align__(16) uint32_t s_mup[SLABW];
+  T neu[CPT];
+  uint32_t nmu[CPT];
+  auto fetch = [&](int64_t slab) {
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) {
+      const int64_t c = slab * SLABW + j * 256 + threadIdx.x;
+      neu[j] = T(0);
+      nmu[j] = 0;
+      if (FIRST && j * 256 + int(threadIdx.x) < SLABW && c < dimup) {
+        neu[j] = a.e_up[c];
+        nmu[j] = a.map_up[c];
+      }
+    }
+  };
+  fetch(0);
   for (int64_t slab = 0; slab < nslab; ++slab) {
     if (threadIdx.x == 0) s_ctr = 0;
-    __syncthreads();
-    const int64_t col0 = slab * (SEGW * NSEG) + int64_t(lane) * EPL;
-    bool act[NSEG];
 #pragma unroll
-    for (int g = 0; g < NSEG; ++g) act[g] = col0 + g * SEGW < dimup;
+    for (int j = 0; j < CPT; ++j)
+      if (FIRST && j * 256 + int(threadIdx.x) < SLABW) {
+        s_eup[j * 256 + threadIdx.x] = neu[j];
+        s_mup[j * 256 + threadIdx.x] = nmu[j];
+      }
+    __syncthreads();
+    fetch(slab + 1);
     for (;;) {
       int rr = 0;
       if (lane == 0) rr = atomicAdd(&s_ctr, 1);
       rr = __shfl_sync(0xffffffffu, rr, 0);
-      if (rr >= nr) break;
+      if (rr >= nr * PARTS) break;
+      int part = 0;
+#pragma unroll
+      for (int j = 1; j < PARTS; ++j) part += rr >= j * nr;
+      rr -= part * nr;
+      const int64_t col0 = slab * SLABW + part * PARTW + int64_t(lane) * EPL;
+      bool act[NSEG];
+#pragma unroll
+      for (int g = 0; g < NSEG; ++g) act[g] = col0 + g * SEGW < dimup;
       const int64_t idw = s_row[rr];
       const T* __restrict__ vrow0 = a.v + col0 * W;   // + src*dimup*W per hop
       const int64_t e0 = idw * dimup + col0;
@@ -789,18 +873,19 @@ __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t*
 #pragma unroll
       for (int g = 0; g < NSEG; ++g) {
         if (!act[g]) continue;
-        const int64_t c = col0 + g * SEGW;
         if (FIRST) {
           const T edw = s_edw[rr];
           const uint32_t mdw = s_mdw[rr];
-          T x[VEC], up[VEC];
+          T x[VEC], up[VEC], eu[EPL];
+          uint32_t mu[EPL];
           VecLd<T, VEC>::load(a.v + (e0 + g * SEGW) * W, x);
+          VecLds<T, EPL>::load(s_eup + part * PARTW + g * SEGW + lane * EPL, eu);
+          VecLds<uint32_t, EPL>::load(s_mup + part * PARTW + g * SEGW + lane * EPL, mu);
           if (SUB) VecLd<T, VEC>::load(a.uprev + e0 + g * SEGW, up);
           const double scl = SCALED ? *static_cast<volatile double*>(&s_sc) : 1.0;
 #pragma unroll
           for (int r = 0; r < VEC; ++r) {
-            const int64_t cr = c + r / W;
-            const T d = a.e_up[cr] + edw + a.U * T(__popc(a.map_up[cr] & mdw));
+            const T d = eu[r / W] + edw + a.U * T(__popc(mu[r / W] & mdw));
             acc[g][r] = (SCALED ? T(double(d) * scl) : d) * x[r];
           }
           if (SUB) {
@@ -810,10 +895,10 @@ __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t*
           }
         } else {
 #pragma unroll
-          for (int r = 0; r < VEC; ++r) acc[g][r] = a.hv[(e0 + g * SEGW) * W + r];
+          for (int r = 0; r < VEC; ++r) acc[g][r] = __ldcs(a.hv + (e0 + g * SEGW) * W + r);
         }
       }
-      for (int k = 0; k < cnt; k += KU) {
+      for (int k = 0; k < cnt; k += KU) {  // reads past the list repeat its batch's first source
         T x[KU][NSEG][VEC];
 #pragma unroll
         for (int u = 0; u < KU; ++u) {
@@ -838,10 +923,7 @@ __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t*
       }
 #pragma unroll
       for (int g = 0; g < NSEG; ++g)
-        if (act[g]) {
-#pragma unroll
-          for (int r = 0; r < VEC; ++r) __stcs(a.hv + (e0 + g * SEGW) * W + r, acc[g][r]);
-        }
+        if (act[g]) VecSt<T, VEC>::store(a.hv + (e0 + g * SEGW) * W, acc[g]);
     }
     __syncthreads();
   }
@@ -855,30 +937,6 @@ __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t*
 // the rank range) reads the source there, every other hop reads it from L2 as k_dw_grp does.
 // The choice is per (row, hop), uniform over the warp, and the terms keep k_dw_grp's order,
 // so results are bit-identical to it.
-template <typename T, int VEC>
-struct VecLds {  // VEC-wide shared-memory load
-  static __device__ __forceinline__ void load(const T* p, T* x) {
-#pragma unroll
-    for (int r = 0; r < VEC; ++r) x[r] = p[r];
-  }
-};
-template <>
-struct VecLds<float, 2> {
-  static __device__ __forceinline__ void load(const float* p, float* x) {
-    const float2 t = *reinterpret_cast<const float2*>(p);
-    x[0] = t.x;
-    x[1] = t.y;
-  }
-};
-template <>
-struct VecLds<double, 2> {
-  static __device__ __forceinline__ void load(const double* p, double* x) {
-    const double2 t = *reinterpret_cast<const double2*>(p);
-    x[0] = t.x;
-    x[1] = t.y;
-  }
-};
-
 template <typename T, int VEC, int NSEG, int KU, bool FIRST, bool SCALED, int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_dw_blk(HxvArgs<T> a, const uint32_t* __restrict__ boff, int64_t nslab) {
   if (!select_column(a)) return;
@@ -1291,19 +1349,27 @@ int launch_up_smem(const HxvArgs<T>& a, const SellArgs<T>& sl, cudaStream_t st, 
   return EDG_OK;
 }
 
-// k_dw_grp over the row groups. FP32: 4 float2 segments per lane (256 columns per slab); FP64: 2
-// double2 segments, 4 hops in flight (3 in the Lanczos-scaled form, which spilled at 4 within
-// the 64 registers of 4 CTAs per SM).
+// k_dw_grp over the row groups, in 2-wide loads where the rows allow it (odd DimUp does not).
+// Hops in flight and slab parts per barrier by type and width, measured in us per H x v:
+//   hops: FP32 2 / 3 / 4: 1564 / 1632 / 1627 on the 4x4 (8,8) sector, 626 / 670 / 665 on (6,6)
+//   (the Lanczos-scaled pass alone there, 2 / 3: 397 / 387);
+//   FP64 2 / 3 / 4: 3187 / 3197 / 3495 and 1259 / 1260 / 1256, odd rows (5x3 (7,8)) 916 / 892 /
+//   1121; odd FP32 rows 3 / 4: 550 / 539. Reads past a list repeat a source and cost L2 -> SM
+//   bandwidth; skipping them (a second, narrower loop) measured slower in every case.
+//   parts 1 / 2 / 4: FP32 1543 / 1611 / 1603, FP64 (6,6) 1236 / 1211 / 1198, (8,8) 3145 / 3141 /
+//   3440; odd rows FP64 890 / 1021 / 1006, FP32 542 / 514 / 502.
+// Narrower slabs (half the segments) cost 15 to 20 %.
 template <typename T, bool FIRST, bool SCALED>
 int launch_dw_grp(const HxvArgs<T>& a, const SpinBasis& Bdw, bool v2, cudaStream_t st) {
-  constexpr int NSEG = sizeof(T) == 4 ? 4 : 2;
-  constexpr int KU = sizeof(T) == 4 ? 3 : (SCALED ? 3 : 4);
-  auto kern = v2 ? k_dw_grp<T, 2, NSEG, KU, FIRST, SCALED> : k_dw_grp<T, 1, NSEG, KU, FIRST, SCALED>;
-  const int vec = v2 ? 2 : 1;
+  constexpr bool F32 = sizeof(T) == 4;
+  constexpr int NSEG = F32 ? 4 : 2;
+  auto kern = v2 ? k_dw_grp<T, 2, NSEG, F32 && !SCALED ? 2 : 3, F32 ? 1 : 2, FIRST, SCALED>
+                 : k_dw_grp<T, 1, 4, F32 ? 4 : 3, F32 ? 2 : 1, FIRST, SCALED>;
   const size_t smem = size_t(Bdw.group_max) * (kDwHops * (sizeof(T) + 4) + sizeof(T) + 12) + 16;
   if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  const int64_t nslab = (a.dimup + 32 * vec * NSEG - 1) / (32 * vec * NSEG);
-  kern<<<dim3(Bdw.groups, a.ncols), 256, smem, st>>>(a, Bdw.group_off.p, Bdw.group_rows.p, nslab, nullptr);
+  const int64_t slab = v2 ? 64 * NSEG * (F32 ? 1 : 2) : 128 * (F32 ? 2 : 1);
+  kern<<<dim3(Bdw.groups, a.ncols), 256, smem, st>>>(a, Bdw.group_off.p, Bdw.group_rows.p, (a.dimup + slab - 1) / slab,
+                                                      nullptr);
   EDG_CUDA(cudaGetLastError());
   return EDG_OK;
 }
@@ -1311,7 +1377,8 @@ int launch_dw_grp(const HxvArgs<T>& a, const SpinBasis& Bdw, bool v2, cudaStream
 // hv += (H_dw x I) v by the row groups.
 template <typename T>
 int dw_add(const HxvArgs<T>& a, const SpinBasis& Bdw, cudaStream_t st) {
-  const bool v2 = a.dimup % 2 == 0 && reinterpret_cast<uintptr_t>(a.v) % (2 * sizeof(T)) == 0;
+  const bool v2 = a.dimup % 2 == 0 && reinterpret_cast<uintptr_t>(a.v) % (2 * sizeof(T)) == 0 &&
+                  reinterpret_cast<uintptr_t>(a.hv) % (2 * sizeof(T)) == 0;
   return launch_dw_grp<T, false, false>(a, Bdw, v2, st);
 }
 
@@ -1356,14 +1423,16 @@ int dw_pass(const HxvArgs<T>& a, const SpinBasis& Bdw, cudaStream_t st, int sms)
   return EDG_OK;
 }
 
-// The down hops of a complex sector (k_dw_grp on complex elements), after diag*v (FIRST) or added to hv.
+// The down hops of a complex sector (k_dw_grp on complex elements), after diag*v (FIRST) or added
+// to hv. 2 hops in flight, 2 parts: 933 us per complex128 H x v of the 4x4 (5,5) sector, against
+// 995 (1 part), 999 (3 hops), 1009 (4 hops).
 template <typename T, bool FIRST>
 int dw_pass_c(const HxvArgs<T>& a, const SpinBasis& Bdw, const T* vi_dw, cudaStream_t st) {
-  constexpr int NSEG = sizeof(T) == 4 ? 4 : 2, KU = sizeof(T) == 4 ? 3 : 4;
-  auto kern = k_dw_grp<T, 2, NSEG, KU, FIRST, false, 2>;
+  constexpr int NSEG = sizeof(T) == 4 ? 4 : 2, PARTS = 2;
+  auto kern = k_dw_grp<T, 2, NSEG, 2, PARTS, FIRST, false, 2>;
   const size_t smem = size_t(Bdw.group_max) * (kDwHops * (2 * sizeof(T) + 4) + sizeof(T) + 12) + 16;
   if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  const int64_t nslab = (a.dimup + 32 * NSEG - 1) / (32 * NSEG);
+  const int64_t slab = 32 * NSEG * PARTS, nslab = (a.dimup + slab - 1) / slab;
   kern<<<dim3(Bdw.groups, 1), 256, smem, st>>>(a, Bdw.group_off.p, Bdw.group_rows.p, nslab, vi_dw);
   EDG_CUDA(cudaGetLastError());
   return EDG_OK;

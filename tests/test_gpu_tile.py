@@ -135,7 +135,7 @@ def flux_lattice(lx, ly, flux):
 
 
 @pytest.mark.parametrize("case", [(8, 1, 0, 4), (8, 1, 4, 0), (3, 3, 4, 5), (11, 1, 5, 4), (3, 4, 6, 5), (7, 2, 7, 3),
-                                  (5, 3, 7, 2), (4, 4, 8, 1), (4, 4, 5, 5)], ids=lambda c: "%dx%d_%d_%d" % c)
+                                  (5, 3, 7, 2), (4, 4, 8, 1), (7, 2, 7, 7)], ids=lambda c: "%dx%d_%d_%d" % c)
 @pytest.mark.parametrize("prec", ["f64", "f32"])
 @pytest.mark.parametrize("form", [E.EDG_FORM_STORED, E.EDG_FORM_DIRECT], ids=["stored", "direct"])
 def test_hxv_tile_complex(case, prec, form):
@@ -143,6 +143,8 @@ def test_hxv_tile_complex(case, prec, form):
     case). FP64 to 1e-13 of the largest element, FP32 to 2e-6."""
     import torch
     lx, ly, nup, ndw = case
+    if nup == ndw == 7 and (prec == "f32") != (form == E.EDG_FORM_DIRECT):
+        pytest.skip("the oracle takes a minute: two passes as stored FP64 and direct FP32 only")
     h = flux_lattice(lx, ly, 0.25)
     s = E.Sector(E.Model(h, uloc=4.0, xmu=2.0, hfmode=False), nup, ndw, form)
     s.set_stream(torch.cuda.current_stream().cuda_stream)
