@@ -312,7 +312,7 @@ int build_spin(edg_sector_s* s, int spin, SpinBasis& B, int nel) {
     if (m.hfmode && m.uloc != 0.0) shift += 0.5 * m.uloc;
   }
   EnergyParams ep{};
-  for (int io = 0; io < ns; ++io) ep.eps[io] = m.hre[sp][io * ns + io] - shift;
+  for (int io = 0; io < ns; ++io) B.eps[io] = ep.eps[io] = m.hre[sp][io * ns + io] - shift;
   EDG_CHECK(B.e64.alloc(B.dim, st, "local energies"));
   EDG_CHECK(B.e32.alloc(B.dim, st, "local energies"));
   {

@@ -124,6 +124,7 @@ struct SpinBasis {
   int nel = 0;                  // Nup or Ndw
   int64_t dim = 0;              // C(Ns, nel)
   DevBuf<uint32_t> map;         // ascending bitstrings [dim]
+  double eps[kMaxSites] = {};   // one-body energies of the sites, shift included
   DevBuf<double> e64;           // local one-body energy of each configuration [dim]
   DevBuf<float> e32;
   // Gather hop table over target rows: row r lists (source rank, value) with
@@ -407,7 +408,6 @@ int scale_into(cudaStream_t st, T* dst, const T* src, const double* b, int64_t n
 template <typename T>
 int lanczos_step_b2(cudaStream_t st, T* w, const T* u, const double* a, const double* bn, int64_t n, double* partial,
                     double* bn_next);
-int finish_dev(cudaStream_t st, const double* partial, int nblk, double* out, int do_sqrt);
 // block forms (ncols columns: vectors vstride elements apart, device scalars sstride apart,
 // reduction scratch kRedSlots apart; columns whose active[c] is 0 are skipped)
 template <typename T>

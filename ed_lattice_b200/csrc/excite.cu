@@ -10,6 +10,8 @@
 //  observables: lanc_observables (src/OBSERVABLES.f90:127-152), per-site moments of |psi|^2.
 // Vectors of a complex-Hij sector hold complex elements interleaved (re, im): the kernels take
 // the element width W (1 real, 2 complex) as a template argument.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace edg {
@@ -163,92 +165,164 @@ __global__ void k_hopop(const double* __restrict__ in, double* __restrict__ out,
   }
 }
 
-// Observables: one CTA per row idw; per-site sums of |psi|^2 weighted by the up bits, then
-// combined with the down bits of the row. out layout per block: [5][kMaxSites].
-template <int W>
-__global__ void __launch_bounds__(256) k_obs_rows(const double* __restrict__ psi, int64_t dup, int64_t ddw,
-                                                  const uint32_t* mup, const uint32_t* mdw, int ns,
-                                                  double* __restrict__ partial) {
-  __shared__ double sq[8][kMaxSites + 1];
-  __shared__ double blk[3][kMaxSites];
-  double acc_up[kMaxSites];
-  double acc_tot = 0.0;
-  for (int i = threadIdx.x; i < 3 * kMaxSites; i += blockDim.x) (&blk[0][0])[i] = 0.0;
+// Observables: per-site sums of |psi|^2. A thread owns C columns (fixed up bits) and walks the
+// rows of its block's chunk: per row one sum for each low site that the row's down configuration
+// occupies (the same test for every thread) and one for all rows since the high half of the
+// configuration changed (rows ascend, so every few tens of rows), which then joins the total and
+// the sums of the high sites it occupies. The up bits enter once, at the end: dens_up_i = sum
+// over columns with bit i of the totals, docc_i the same of the site sums, dens_dw_i the site
+// sums over all columns. One row per CTA with a test and a 64-bit select for each of 30 sites
+// and element took 1205 us on the 4x4 (7,7) sector (1.05 GB). partial[block][3][kMaxSites].
+template <int NS, int W, int C>
+__global__ void __launch_bounds__(256) k_obs_cols(const double* __restrict__ psi, int64_t dup, int64_t ddw,
+                                                  const uint32_t* __restrict__ mup, const uint32_t* __restrict__ mdw,
+                                                  int rows_per, double* __restrict__ partial) {
+  extern __shared__ uint32_t s_md[];
+  __shared__ double s_sum[8][3 * NS];
+  const int64_t r0 = int64_t(blockIdx.y) * rows_per;
+  const int nr = int(ddw - r0 < rows_per ? ddw - r0 : rows_per);
+  for (int i = threadIdx.x; i < nr; i += blockDim.x) s_md[i] = mdw[r0 + i];
   __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int64_t row = blockIdx.x; row < ddw; row += gridDim.x) {
+  constexpr int M = NS / 2;  // low sites
+  double tot[C], blk[C], x[C][NS];
+  int64_t col[C];
 #pragma unroll
-    for (int i = 0; i < kMaxSites; ++i) acc_up[i] = 0.0;
-    acc_tot = 0.0;
-    for (int64_t j = threadIdx.x; j < dup; j += blockDim.x) {
-      const double p = psi[(row * dup + j) * W];
-      const double q = psi[(row * dup + j) * W + W - 1];
-      const double w = W == 1 ? p * p : __fma_rn(q, q, p * p);
-      const uint32_t u = mup[j];
-      acc_tot += w;
+  for (int k = 0; k < C; ++k) {
+    col[k] = int64_t(blockIdx.x) * (256 * C) + k * 256 + threadIdx.x;
+    tot[k] = blk[k] = 0.0;
 #pragma unroll
-      for (int i = 0; i < kMaxSites; ++i) acc_up[i] += ((u >> i) & 1u) ? w : 0.0;
-    }
-    // block reduce (kMaxSites + 1 values)
+    for (int i = 0; i < NS; ++i) x[k][i] = 0.0;
+  }
+  uint32_t high = s_md[0] >> M;  // the rows' high part; blk sums the rows since it changed
+  auto flush = [&] {
 #pragma unroll
-    for (int i = 0; i <= kMaxSites; ++i) {
-      double v = i < kMaxSites ? acc_up[i] : acc_tot;
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0) sq[wid][i] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const uint32_t d = mdw[row];
-      double tot = 0.0;
-      for (int w8 = 0; w8 < 8; ++w8) tot += sq[w8][kMaxSites];
-      for (int i = 0; i < ns; ++i) {
-        double qu = 0.0;
-        for (int w8 = 0; w8 < 8; ++w8) qu += sq[w8][i];
-        const double nd = double((d >> i) & 1u);
-        blk[0][i] += qu;
-        blk[1][i] += nd * tot;
-        blk[2][i] += nd * qu;
+    for (int i = M; i < NS; ++i)
+      if ((high >> (i - M)) & 1u) {
+#pragma unroll
+        for (int k = 0; k < C; ++k) x[k][i] += blk[k];
       }
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+      tot[k] += blk[k];
+      blk[k] = 0.0;
     }
-    __syncthreads();
+  };
+  constexpr int U = 4;  // rows whose elements are loaded together
+  for (int r = 0; r < nr; r += U) {
+    double p[U][C], q[U][C];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < C; ++k) {
+        p[u][k] = q[u][k] = 0.0;
+        if (r + u < nr && col[k] < dup) {
+          const double* e = psi + ((r0 + r + u) * dup + col[k]) * W;
+          p[u][k] = __ldcs(e);
+          if (W == 2) q[u][k] = __ldcs(e + W - 1);
+        }
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t d = s_md[min(r + u, nr - 1)];  // past the chunk: zero elements of its last row
+      if ((d >> M) != high) {
+        flush();
+        high = d >> M;
+      }
+      double w[C];
+#pragma unroll
+      for (int k = 0; k < C; ++k) {
+        w[k] = W == 1 ? p[u][k] * p[u][k] : __fma_rn(q[u][k], q[u][k], p[u][k] * p[u][k]);
+        blk[k] += w[k];
+      }
+#pragma unroll
+      for (int i = 0; i < M; ++i)
+        if ((d >> i) & 1u) {
+#pragma unroll
+          for (int k = 0; k < C; ++k) x[k][i] += w[k];
+        }
+    }
   }
+  flush();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint32_t up[C];
+#pragma unroll
+  for (int k = 0; k < C; ++k) up[k] = col[k] < dup ? mup[col[k]] : 0u;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) {
+    double v[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+      const bool on = (up[k] >> i) & 1u;
+      v[0] += on ? tot[k] : 0.0;
+      v[1] += x[k][i];
+      v[2] += on ? x[k][i] : 0.0;
+    }
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      for (int o = 16; o > 0; o >>= 1) v[t] += __shfl_down_sync(0xffffffffu, v[t], o);
+      if (lane == 0) s_sum[wid][t * NS + i] = v[t];
+    }
+  }
+  __syncthreads();
+  double* out = partial + (int64_t(blockIdx.y) * gridDim.x + blockIdx.x) * 3 * kMaxSites;
+  for (int j = threadIdx.x; j < 3 * NS; j += blockDim.x)
+    if (j % NS < kMaxSites) {
+      double t = 0.0;
+      for (int w = 0; w < 8; ++w) t += s_sum[w][j];
+      out[j / NS * kMaxSites + j % NS] = t;
+    }
+}
+
+// out[v] = sum over blocks of partial[block][v], v < gridDim.x, fixed order
+__global__ void __launch_bounds__(256) k_obs_sum(const double* __restrict__ partial, int nblk, double* __restrict__ out) {
+  __shared__ double sh[8];
+  double t = 0.0;
+  for (int b = threadIdx.x; b < nblk; b += 256) t += partial[int64_t(b) * 3 * kMaxSites + blockIdx.x];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+  __syncthreads();
   if (threadIdx.x == 0) {
-    double* o = partial + int64_t(blockIdx.x) * 3 * kMaxSites;
-    for (int i = 0; i < kMaxSites; ++i) {
-      o[i] = blk[0][i];
-      o[kMaxSites + i] = blk[1][i];
-      o[2 * kMaxSites + i] = blk[2][i];
-    }
+    t = 0.0;
+    for (int w = 0; w < 8; ++w) t += sh[w];
+    out[blockIdx.x] = t;
   }
+}
+
+template <int NS, int W>
+int launch_obs(const edg_sector_s* s, const double* psi, DevBuf<double>& part, double* sums, cudaStream_t st) {
+  constexpr int C = NS <= 16 ? 2 : 1;
+  const int64_t gx = (s->up.dim + 256 * C - 1) / (256 * C);
+  // about 8 blocks per SM, at least 8 rows each (the closing reduction costs as much as 10 rows)
+  int64_t gy = std::max<int64_t>(1, std::min<int64_t>((s->dw.dim + 7) / 8, (148 * 8 + gx - 1) / gx));
+  int64_t per = (s->dw.dim + gy - 1) / gy;
+  if (per > 10240) per = 10240;  // row masks in shared memory
+  gy = (s->dw.dim + per - 1) / per;
+  const int64_t nblk = gx * gy;
+  EDG_CHECK(part.alloc(size_t(nblk + 1) * 3 * kMaxSites, st, "observable partials"));
+  EDG_CUDA(cudaMemsetAsync(part.p, 0, size_t(nblk + 1) * 3 * kMaxSites * sizeof(double), st));
+  k_obs_cols<NS, W, C><<<dim3(unsigned(gx), unsigned(gy)), 256, size_t(per) * sizeof(uint32_t), st>>>(
+      psi, s->up.dim, s->dw.dim, s->up.map.p, s->dw.map.p, int(per), part.p);
+  double* out = part.p + size_t(nblk) * 3 * kMaxSites;
+  k_obs_sum<<<3 * kMaxSites, 256, 0, st>>>(part.p, int(nblk), out);
+  EDG_CUDA(cudaGetLastError());
+  EDG_CUDA(cudaMemcpyAsync(sums, out, 3 * kMaxSites * sizeof(double), cudaMemcpyDeviceToHost, st));
+  EDG_CUDA(cudaStreamSynchronize(st));
+  return EDG_OK;
+}
+
+// sums[0][i], [1][i], [2][i]: up density, down density and double occupancy of site i in psi
+template <int W>
+int site_sums(const edg_sector_s* s, const double* psi, double (*sums)[kMaxSites], cudaStream_t st) {
+  DevBuf<double> part;
+  const int ns = s->model.ns;
+  if (ns <= 8) return launch_obs<8, W>(s, psi, part, sums[0], st);
+  if (ns <= 12) return launch_obs<12, W>(s, psi, part, sums[0], st);
+  if (ns <= 16) return launch_obs<16, W>(s, psi, part, sums[0], st);
+  if (ns <= 20) return launch_obs<20, W>(s, psi, part, sums[0], st);
+  return launch_obs<32, W>(s, psi, part, sums[0], st);
 }
 
 int grid_rows(int64_t rows) { return int(rows < 148 * 8 ? (rows < 1 ? 1 : rows) : 148 * 8); }
-
-// Partial sums of psi_i^2 diag(H)_i with diag(H)_i = E_up[iup] + E_dw[idw] + U popc(up & dw),
-// the diagonal the H x v applies; fixed grid and order (deterministic).
-constexpr int kDiagBlocks = 592;
-template <int W>
-__global__ void __launch_bounds__(256) k_diag_dot(const double* __restrict__ psi, int64_t dup, int64_t n,
-                                                  const double* __restrict__ eup, const double* __restrict__ edw,
-                                                  const uint32_t* __restrict__ mup, const uint32_t* __restrict__ mdw,
-                                                  double U, double* __restrict__ partial) {
-  __shared__ double sh[8];
-  double s = 0.0;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t idw = i / dup, iup = i - idw * dup;
-    const double d = eup[iup] + edw[idw] + U * double(__popc(mup[iup] & mdw[idw]));
-    const double p = psi[i * W], q = psi[i * W + W - 1];
-    s = __fma_rn(W == 1 ? p * p : __fma_rn(q, q, p * p), d, s);
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < int(blockDim.x >> 5); ++w) t += sh[w];
-    partial[blockIdx.x] = t;
-  }
-}
 
 }  // namespace
 
@@ -346,25 +420,10 @@ int apply_current(const edg_sector_s* s, const double* din, double* dout, cudaSt
 
 int observables(const edg_sector_s* s, const double* psi, double weight, double* dens, double* dens_up,
                 double* dens_dw, double* docc, double* magz, cudaStream_t st) {
-  const int ns = s->model.ns;
-  const int g = grid_rows(s->dw.dim);
-  DevBuf<double> part;
-  EDG_CHECK(part.alloc(size_t(g) * 3 * kMaxSites, st, "observable partials"));
-  if (s->cplx)
-    k_obs_rows<2><<<g, 256, 0, st>>>(psi, s->up.dim, s->dw.dim, s->up.map.p, s->dw.map.p, ns, part.p);
-  else
-    k_obs_rows<1><<<g, 256, 0, st>>>(psi, s->up.dim, s->dw.dim, s->up.map.p, s->dw.map.p, ns, part.p);
-  EDG_CUDA(cudaGetLastError());
-  std::vector<double> h(size_t(g) * 3 * kMaxSites);
-  EDG_CUDA(cudaMemcpyAsync(h.data(), part.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-  EDG_CUDA(cudaStreamSynchronize(st));
-  for (int i = 0; i < ns; ++i) {
-    double u = 0, d = 0, dd = 0;
-    for (int b = 0; b < g; ++b) {
-      u += h[size_t(b) * 3 * kMaxSites + i];
-      d += h[size_t(b) * 3 * kMaxSites + kMaxSites + i];
-      dd += h[size_t(b) * 3 * kMaxSites + 2 * kMaxSites + i];
-    }
+  double q[3][kMaxSites];
+  EDG_CHECK(s->cplx ? site_sums<2>(s, psi, q, st) : site_sums<1>(s, psi, q, st));
+  for (int i = 0; i < s->model.ns; ++i) {
+    const double u = q[0][i], d = q[1][i], dd = q[2][i];
     if (dens_up) dens_up[i] += weight * u;
     if (dens_dw) dens_dw[i] += weight * d;
     if (dens) dens[i] += weight * (u + d);
@@ -375,7 +434,9 @@ int observables(const edg_sector_s* s, const double* psi, double weight, double*
 }
 
 // lanc_energy (src/ENERGY.f90:118-226, Norb=1 terms) for one state:
-//  ekin = <psi|H|psi> - <psi|diag(H)|psi> (the off-diagonal part is exactly the hopping),
+//  ekin = <psi|H|psi> - <psi|diag(H)|psi> (the off-diagonal part is exactly the hopping), with
+//  diag(H) from the site sums: sum_i eps_i n_i per spin + U docc_i, eps_i the one-body energies
+//  that the H x v applies (SpinBasis::eps),
 //  eknot from the Hij diagonal and the site densities, epot = U sum_i docc_i plus the Hartree
 //  term -U/2 sum_i n_i when HFMODE (reported also on its own, as ENERGY.f90:343 adds it).
 int energy(edg_sector_s* s, const double* psi, double weight, double* ekin, double* epot, double* eknot,
@@ -383,36 +444,36 @@ int energy(edg_sector_s* s, const double* psi, double weight, double* ekin, doub
   const int ns = s->model.ns;
   const int64_t n = s->vlen;  // <psi|H psi> over reals = Re <psi|H|psi> for complex psi
   cudaStream_t st = s->stream;
-  std::vector<double> dens(ns, 0.0), nup(ns, 0.0), ndw(ns, 0.0), docc(ns, 0.0);
-  EDG_CHECK(observables(s, psi, 1.0, dens.data(), nup.data(), ndw.data(), docc.data(), nullptr, st));
   EDG_CHECK(s->w64[0].alloc(n, st, "energy work vector"));
   double* hv = s->w64[0].p;
-  EDG_CHECK(hxv_apply<double>(s, psi, hv));
   DevBuf<double> part;
-  EDG_CHECK(part.alloc(size_t(kRedSlots) + kDiagBlocks + 4, st, "energy partials"));
-  double* out = part.p + kRedSlots + kDiagBlocks;
+  EDG_CHECK(part.alloc(size_t(kRedSlots) + 4, st, "energy partials"));
+  double* out = part.p + kRedSlots;
   EDG_CHECK(red_scratch_reset(st, part.p));
-  EDG_CHECK(dot_dev<double>(st, psi, hv, n, part.p, out));
-  if (s->cplx)
-    k_diag_dot<2><<<kDiagBlocks, 256, 0, st>>>(psi, s->up.dim, s->dim, s->up.e64.p, s->dw.e64.p, s->up.map.p,
-                                               s->dw.map.p, s->U, part.p + kRedSlots);
-  else
-    k_diag_dot<1><<<kDiagBlocks, 256, 0, st>>>(psi, s->up.dim, s->dim, s->up.e64.p, s->dw.e64.p, s->up.map.p,
-                                               s->dw.map.p, s->U, part.p + kRedSlots);
-  EDG_CUDA(cudaGetLastError());
-  EDG_CHECK(finish_dev(st, part.p + kRedSlots, kDiagBlocks, out + 1, 0));
-  double h[2] = {0.0, 0.0};
-  EDG_CUDA(cudaMemcpyAsync(h, out, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
-  EDG_CUDA(cudaStreamSynchronize(st));
+  if (hxv_lz_available(s, sizeof(double))) {
+    // the Lanczos-fused product at step 0 with unit scale: w = H psi - 0 * psi and <psi, w>
+    const double one = 1.0;
+    EDG_CUDA(cudaMemcpyAsync(out + 1, &one, sizeof(double), cudaMemcpyHostToDevice, st));
+    EDG_CHECK(hxv_apply_lz<double>(s, psi, psi, hv, out + 1, 0, part.p, out));
+  } else {
+    EDG_CHECK(hxv_apply<double>(s, psi, hv));
+    EDG_CHECK(dot_dev<double>(st, psi, hv, n, part.p, out));
+  }
+  double h = 0.0;
+  EDG_CUDA(cudaMemcpyAsync(&h, out, sizeof(double), cudaMemcpyDeviceToHost, st));
+  double q[3][kMaxSites];  // (the site sums wait for the stream: h and `one` are settled after)
+  EDG_CHECK(s->cplx ? site_sums<2>(s, psi, q, st) : site_sums<1>(s, psi, q, st));
   const std::vector<double>& h1 = s->model.hre[0];
   const std::vector<double>& h2 = s->model.nspin == 2 ? s->model.hre[1] : s->model.hre[0];
-  double kn = 0.0, ep = 0.0, eh = 0.0;
+  double kn = 0.0, ep = 0.0, eh = 0.0, dg = 0.0;
   for (int i = 0; i < ns; ++i) {
-    kn += h1[size_t(i) * ns + i] * nup[i] + h2[size_t(i) * ns + i] * ndw[i];
-    ep += s->model.uloc * docc[i];
-    if (s->model.hfmode) eh -= 0.5 * s->model.uloc * dens[i];
+    const double nu = q[0][i], nd = q[1][i], dd = q[2][i];
+    kn += h1[size_t(i) * ns + i] * nu + h2[size_t(i) * ns + i] * nd;
+    ep += s->model.uloc * dd;
+    dg += s->up.eps[i] * nu + s->dw.eps[i] * nd + s->U * dd;
+    if (s->model.hfmode) eh -= 0.5 * s->model.uloc * (nu + nd);
   }
-  if (ekin) *ekin += weight * (h[0] - h[1]);
+  if (ekin) *ekin += weight * (h - dg);
   if (eknot) *eknot += weight * kn;
   if (epot) *epot += weight * (ep + eh);
   if (ehartree) *ehartree += weight * eh;

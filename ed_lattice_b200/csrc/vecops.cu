@@ -77,15 +77,6 @@ __global__ void __launch_bounds__(kRedThreads) k_dot(const T* __restrict__ x, co
   finish_in_last_block(partial, gridDim.x, out, do_sqrt);
 }
 
-// out = sum(partial) (do_sqrt: sqrt of the sum)
-__global__ void __launch_bounds__(kRedThreads) k_finish(const double* __restrict__ partial, int nblk,
-                                                        double* __restrict__ out, int do_sqrt) {
-  double s = 0.0;
-  for (int i = threadIdx.x; i < nblk; i += blockDim.x) s += partial[i];
-  s = block_sum(s);
-  if (threadIdx.x == 0) out[0] = do_sqrt ? sqrt(s) : s;
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads) k_step_a(T* __restrict__ w, const T* __restrict__ vprev,
                                                         const T* __restrict__ v, const double* __restrict__ bprev,
@@ -502,12 +493,6 @@ int norm_dev(cudaStream_t st, const double* x, int64_t n, double* partial, doubl
 
 int red_scratch_reset(cudaStream_t st, double* partial) {
   EDG_CUDA(cudaMemsetAsync(partial + kRedMaxBlocks, 0, sizeof(double), st));
-  return EDG_OK;
-}
-
-int finish_dev(cudaStream_t st, const double* partial, int nblk, double* out, int do_sqrt) {
-  k_finish<<<1, kRedThreads, 0, st>>>(partial, nblk, out, do_sqrt);
-  EDG_CUDA(cudaGetLastError());
   return EDG_OK;
 }
 
