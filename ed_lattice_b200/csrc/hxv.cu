@@ -1598,7 +1598,7 @@ HxvArgs<T> make_args(edg_sector_s* s, const T* v, T* hv) {
 // By row tiles (tile.cu) where the tile kernels apply, else the per-column gathers.
 template <typename T, bool LZ>
 int fused_pass(edg_sector_s* s, const HxvArgs<T>& a, cudaStream_t st, int sms) {
-  if (tile_available(s, sizeof(T), true) && s->dim >= kTileMinDim)
+  if (tile_available(s, sizeof(T), true) && s->dim >= (sizeof(T) == 8 ? kTileMinDim64 : kTileMinDim32))
     return tile_real<T>(a, s->up, s->dw, TileForm::kDwUp, LZ, st, sms);
   const int64_t ntiles = a.dimdw * ((a.dimup + 31) / 32);
   const int64_t want = (ntiles + 7) / 8;

@@ -169,6 +169,31 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
     const int rows = int(a.dimdw - r0 < RT ? a.dimdw - r0 : RT);
     const E* __restrict__ vt = reinterpret_cast<const E*>(a.v) + r0 * dimup;
     E* __restrict__ ht = reinterpret_cast<E*>(a.hv) + r0 * dimup;
+    // The first entries, (rows-in form) sums and (down form) diagonal terms of each slice are
+    // loaded while the slice before it runs, the first one's while the tile is staged.
+    int sl = s0 + warp;
+    uint32_t o = 0, o1 = 0;
+    uint4 b0 = make_uint4(0u, 0u, 0u, 0u);
+    uint2 c0 = make_uint2(0u, 0u);
+    E hn[RT] = {};
+    T eun = T(0);
+    uint32_t mun = 0;
+    if (sl < s1) {
+      const uint32_t w = q.off[sl];
+      o = (w >> 9) * 2;
+      o1 = o + (w & 511u);
+      b0 = __ldg(q.ent + o * 16u + lane);
+      if (PAL) c0 = __ldg(q.code + o * 16u + lane);
+      const int c = min(sl * 32 + lane, dimup - 1);
+      if (DIAG) {
+        eun = a.e_up[c];
+        mun = a.map_up[c];
+      } else {
+#pragma unroll
+        for (int r = 0; r < RT; ++r)
+          if (r < rows) hn[r] = ht[r * dimup + c];
+      }
+    }
 #pragma unroll 7
     for (int j = threadIdx.x; j < dimup; j += blockDim.x) {
       ulonglong2 slot = make_ulonglong2(0, 0);
@@ -198,31 +223,6 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
       }
     }
     __syncthreads();
-    // The first entries, (rows-in form) sums and (down form) diagonal terms of each slice are
-    // loaded while the slice before it runs.
-    int sl = s0 + warp;
-    uint32_t o = 0, o1 = 0;
-    uint4 b0 = make_uint4(0u, 0u, 0u, 0u);
-    uint2 c0 = make_uint2(0u, 0u);
-    E hn[RT] = {};
-    T eun = T(0);
-    uint32_t mun = 0;
-    if (sl < s1) {
-      const uint32_t w = s_off[sl];
-      o = (w >> 9) * 2;
-      o1 = o + (w & 511u);
-      b0 = __ldg(q.ent + o * 16u + lane);
-      if (PAL) c0 = __ldg(q.code + o * 16u + lane);
-      const int c = min(sl * 32 + lane, dimup - 1);
-      if (DIAG) {
-        eun = a.e_up[c];
-        mun = a.map_up[c];
-      } else {
-#pragma unroll
-        for (int r = 0; r < RT; ++r)
-          if (r < rows) hn[r] = ht[r * dimup + c];
-      }
-    }
     while (sl < s1) {
       const int iup = sl * 32 + lane;
       const bool act = iup < dimup;
@@ -402,16 +402,24 @@ int launch(const HxvArgs<T>& a, TileArgs<T, W>& q, cudaStream_t st, int sms) {
   if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   // 64 registers a thread: 1024 threads per SM, in as many CTAs as the tiles leave room for
   const int per_sm = smem <= 54 * 1024 ? 4 : smem <= 111 * 1024 ? 2 : 1;
-  const int threads = 1024 / per_sm;
   q.nsl = int((a.dimup + 31) / 32);
   q.ntile = int((a.dimdw + RT - 1) / RT);
-  // whole product of a sector with few tiles: column parts of a tile, each staging the whole
-  // rows again, until three quarters of the resident CTAs have one (3x4 lattice, D = 853,776,
-  // one part against two: FP32, 231 tiles, 20.8 against 17.6 us; FP64, 462 tiles, 24.1 against
-  // 23.1, with four 26)
-  const int want = (3 * sms * per_sm / 4 + q.ntile - 1) / q.ntile;
-  const int most = std::max(1, q.nsl / (threads / 32));
-  q.csplit = DOWN ? std::max(1, std::min(want, most)) : 1;
+  int warps = 32 / per_sm;
+  q.csplit = 1;
+  if (DOWN) {
+    // Whole product of a sector with few tiles: column parts of a tile, each staging the whole
+    // rows again. With fewer slices than resident warps each warp gets one; else parts until
+    // three quarters of the resident CTAs have one (3x4 lattice, D = 853,776, one part against
+    // two: FP32, 231 tiles, 20.8 against 17.6 us; FP64, 462 tiles, 24.1 against 23.1, with four
+    // 26). The CTA then takes no more warps than its rounds of slices fill.
+    if (int64_t(q.ntile) * q.nsl <= int64_t(sms) * 32)
+      q.csplit = (q.nsl + warps - 1) / warps;
+    else
+      q.csplit = std::max(1, std::min((3 * sms * per_sm / 4 + q.ntile - 1) / q.ntile, q.nsl / warps));
+    const int most = (q.nsl + q.csplit - 1) / q.csplit, rounds = (most + warps - 1) / warps;
+    warps = (most + rounds - 1) / rounds;
+  }
+  const int threads = 32 * warps;
   int64_t g = int64_t(q.ntile) * q.csplit;
   if (!DOWN || g > kRedMaxBlocks) g = std::min<int64_t>(g, DOWN ? kRedMaxBlocks : int64_t(sms) * per_sm);
   kern<<<dim3(unsigned(g), a.ncols), threads, smem, st>>>(a, q);

@@ -35,7 +35,9 @@ CASES = [
     (8, 1, 4, 0, 0.0),    # one row
     (8, 1, 1, 7, 0.0),    # 8 columns, 8 rows
     (3, 3, 4, 5, 0.0),    # 126 x 126: part slices, even rows
-    (11, 1, 5, 4, 0.0),   # 462 x 330: single pass by tiles
+    (11, 1, 5, 4, 0.0),   # 462 x 330: single pass by tiles in FP64
+    (11, 1, 5, 5, 0.0),   # 462 x 462: and in FP32
+    (13, 1, 3, 3, 0.125),  # 286 x 286: nine slices, fewer than the resident warps
     (3, 4, 1, 6, 0.0),    # 12 x 924: a third of a slice, many tiles
     (3, 4, 6, 1, 0.0),    # 924 x 12: few tiles, column parts
     (3, 4, 5, 6, 0.25),   # 792 x 924, two hopping values
