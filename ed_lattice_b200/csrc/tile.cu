@@ -27,6 +27,7 @@
 //   complex128 4x4 (5,5): 2433 (one thread per element, L1 gathers) -> 1157 in two passes;
 //   3x4 (6,6) 81 -> 44, 4x4 (4,5) 825 -> 326 in one launch
 #include <algorithm>
+#include <type_traits>
 
 #include "hxv.cuh"
 #include "reduce.cuh"
@@ -41,6 +42,7 @@ struct TileArgs {
   const uint32_t* __restrict__ off;    // [nsl] first batch of a slice << 9 | its half batches (four slots)
   const double* __restrict__ pal;      // palette: W doubles per code (PAL)
   T h;                                 // value of sign bit 0 (!PAL)
+  T h_dw = T(0);                       // the same of the down hops
   int npal = 0;
   int nsl = 0, ntile = 0;
   int csplit = 1;                      // column parts of a tile, each its own work item
@@ -116,7 +118,10 @@ __device__ __forceinline__ void elem_fma(const T* h, const T* x, T* acc) {
   else cmad(h[0], h[1], x, acc);
 }
 
-// A down hop of a row: the value and the first element of the source row.
+// A down hop of a row: the value and the first element of the source row. The plain product over
+// tables of one |value| keeps the element with the value's sign in bit 31 instead (PACK): four
+// hops per shared-memory load (3x4 (6,6) FP64 22.3 -> 20.4 us). The Lanczos-fused one, short of
+// registers, is slower with it (12 columns of 731,808: 202 -> 217 us).
 template <typename T, int W>
 struct alignas(8) Hop {
   T val[W];
@@ -134,7 +139,8 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
   // uprev is subtracted here, after all hops, unless the down pass began from -c * uprev
   constexpr bool SUB = LZ && (DOWN || !lz_sub_in_dw<T>());
   using E = Elem<T, W>;
-  using H = Hop<T, W>;
+  constexpr bool PACK = !PAL && !LZ;  // packed down hops
+  using H = std::conditional_t<PACK, uint32_t, Hop<T, W>>;
   extern __shared__ __align__(16) unsigned char smem_tile[];
   const int dimup = int(a.dimup);
   ulonglong2* S = reinterpret_cast<ulonglong2*>(smem_tile);
@@ -209,11 +215,16 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
         if (r >= rows) break;
         const uint32_t k0 = a.off_dw[r0 + r], n = a.off_dw[r0 + r + 1] - k0;
         for (uint32_t k = threadIdx.x; DOWN && k < n; k += blockDim.x) {
-          H h;
-          h.val[0] = LZ ? T(double(a.val_dw[k0 + k]) * sc) : a.val_dw[k0 + k];
-          if (W == 2) h.val[W - 1] = q.vi_dw[k0 + k];
-          h.src = a.src_dw[k0 + k] * uint32_t(dimup);
-          l_hop[r * q.cap + k] = h;
+          const uint32_t src = a.src_dw[k0 + k] * uint32_t(dimup);
+          if constexpr (!PACK) {
+            H h;
+            h.val[0] = LZ ? T(double(a.val_dw[k0 + k]) * sc) : a.val_dw[k0 + k];
+            if (W == 2) h.val[W - 1] = q.vi_dw[k0 + k];
+            h.src = src;
+            l_hop[r * q.cap + k] = h;
+          } else {
+            l_hop[r * q.cap + k] = src | (a.val_dw[k0 + k] == q.h_dw ? 0u : 0x80000000u);
+          }
         }
         if (threadIdx.x == 0) {
           s_edw[r] = a.e_dw[r0 + r];
@@ -248,11 +259,19 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
         if (lane < 8 && sl - s0 >= half && nr0 + pr < a.dimdw && pc < dimup)
           asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const E*>(a.v) + (nr0 + pr) * dimup + pc));
       }
+      // uprev: read here next to the down hops; in the up pass fetched into L2 here and read at
+      // the end (4x4 (6,6) 818 -> 794 us; the other way round each is slower)
       T up[RT];
-      if (LZ) {
+      if (SUB && DOWN) {
 #pragma unroll
         for (int r = 0; r < RT; ++r)
-          if (SUB && r < rows) up[r] = a.uprev[(r0 + r) * dimup + c];
+          if (r < rows) up[r] = a.uprev[(r0 + r) * dimup + c];
+      }
+      if (SUB && !DOWN) {
+        constexpr int kLine = 128 / int(sizeof(T)), kPer = 32 / kLine;  // columns per line, lines per row
+        const int pr = lane / kPer, pc = sl * 32 + lane % kPer * kLine;
+        if (pr < rows && pc < dimup)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(a.uprev + (r0 + pr) * dimup + pc));
       }
       // acc += the down hops of the tile's rows
       auto down_hops = [&](T* acc) {
@@ -263,20 +282,51 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
           const int n = s_cnt[r];
           const H* lh = l_hop + r * q.cap;
           int k = 0;
-          for (; k + KU <= n; k += KU) {  // KU independent source reads, then their terms in order
-            E x[KU];
+          if constexpr (PACK) {
+            // K independent source reads, then their terms in order
+            auto batch = [&](auto num, const uint32_t* e, int left) {
+              constexpr int K = decltype(num)::value;
+              E x[K];
 #pragma unroll
-            for (int u = 0; u < KU; ++u) x[u] = vc[lh[k + u].src];
+              for (int u = 0; u < K; ++u)
+                if (K > 3 || u < left) x[u] = vc[e[u] & 0x7fffffffu];
 #pragma unroll
-            for (int u = 0; u < KU; ++u) elem_fma<T, W>(lh[k + u].val, x[u].x, acc + r * W);
-          }
-          if (k < n) {  // the rest: reads past the list repeat its last source
-            E x[KU];
+              for (int u = 0; u < K; ++u)
+                if (K > 3 || u < left) acc[r] = fmaT<T>(flip_sign(q.h_dw, e[u]), x[u].x[0], acc[r]);
+            };
+            const uint4* l4 = reinterpret_cast<const uint4*>(lh);
+            for (; k + 8 <= n; k += 8) {
+              const uint4 e0 = l4[k >> 2], e1 = l4[(k >> 2) + 1];
+              const uint32_t e[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+              batch(std::integral_constant<int, 8>{}, e, 8);
+            }
+            if (k + 4 <= n) {
+              const uint4 e0 = l4[k >> 2];
+              const uint32_t e[4] = {e0.x, e0.y, e0.z, e0.w};
+              batch(std::integral_constant<int, 4>{}, e, 4);
+              k += 4;
+            }
+            if (k < n) {
+              const uint4 e0 = l4[k >> 2];
+              const uint32_t e[3] = {e0.x, e0.y, e0.z};
+              batch(std::integral_constant<int, 3>{}, e, n - k);
+            }
+          } else {
+            for (; k + KU <= n; k += KU) {  // KU independent source reads, then their terms in order
+              E x[KU];
 #pragma unroll
-            for (int u = 0; u < KU - 1; ++u) x[u] = vc[lh[min(k + u, n - 1)].src];
+              for (int u = 0; u < KU; ++u) x[u] = vc[lh[k + u].src];
 #pragma unroll
-            for (int u = 0; u < KU - 1; ++u)
-              if (k + u < n) elem_fma<T, W>(lh[k + u].val, x[u].x, acc + r * W);
+              for (int u = 0; u < KU; ++u) elem_fma<T, W>(lh[k + u].val, x[u].x, acc + r * W);
+            }
+            if (k < n) {  // the rest: reads past the list repeat its last source
+              E x[KU];
+#pragma unroll
+              for (int u = 0; u < KU - 1; ++u) x[u] = vc[lh[min(k + u, n - 1)].src];
+#pragma unroll
+              for (int u = 0; u < KU - 1; ++u)
+                if (k + u < n) elem_fma<T, W>(lh[k + u].val, x[u].x, acc + r * W);
+            }
           }
         }
       };
@@ -339,6 +389,11 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
           }
           acc.fma(h, x);
         }
+      }
+      if (SUB && !DOWN) {
+#pragma unroll
+        for (int r = 0; r < RT; ++r)
+          if (r < rows) up[r] = a.uprev[(r0 + r) * dimup + c];
       }
       T res[N];
 #pragma unroll
@@ -446,7 +501,8 @@ int tile_pass(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, con
   q.pal = up.t16_pal.p;
   q.h = T(up.sell_h);
   q.npal = up.t16_npal;
-  q.cap = form == TileForm::kDwUp || form == TileForm::kUpDw ? dw.max_row : 0;
+  q.h_dw = T(dw.sell_h);
+  q.cap = form == TileForm::kDwUp || form == TileForm::kUpDw ? (dw.max_row + 3) / 4 * 4 : 0;
   q.vi_dw = vi_dw;
   if constexpr (W == 1) {
     if (lz)
@@ -467,7 +523,9 @@ bool tile_available(const edg_sector_s* s, size_t elem, bool down) {
   const SpinBasis& up = s->up;
   if (!up.t16) return false;
   const int rt = int(16 / elem);  // elem: bytes per vector element (a complex one counts whole)
-  return tile_smem(up.dim, up.t16_npal, down ? rt * s->dw.max_row : 0, elem) <= kTileSmemMax;
+  // the single-value form of the whole product needs one |value| on either side
+  if (down && up.t16_npal == 0 && !s->dw.sell_uniform) return false;
+  return tile_smem(up.dim, up.t16_npal, down ? rt * ((s->dw.max_row + 3) / 4 * 4) : 0, elem) <= kTileSmemMax;
 }
 
 template <typename T>
