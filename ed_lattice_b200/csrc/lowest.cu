@@ -257,24 +257,60 @@ __global__ void __launch_bounds__(kLkThreads) k_multiaxpy(const TQ* __restrict__
   }
 }
 
-// X[r][i] = sum_j Z[j*m + r] Q[j][i], r < k (Z column-major m x m, first k columns)
-template <typename TQ>
-__global__ void __launch_bounds__(kLkThreads) k_ritz_k(const TQ* __restrict__ Q, const double* __restrict__ Z,
-                                                       int m, int k, int64_t n, double* __restrict__ X) {
+// X[r][i] = sum_j Z[j + r*m] Q[j][i], r < k <= K, the coefficients in shared memory ([j][K], so a
+// thread's K of a column are neighbours). X may be Q itself: a thread reads all of its element's
+// columns before it writes them, so a restart replaces the basis by its Ritz vectors in place
+// (40 columns of 853,776 to 13 vectors: 91 us; with the coefficients read from global memory, a
+// buffer and copies back, 208 + 13 x 5 us).
+template <typename TQ, typename TX, int K>
+__global__ void __launch_bounds__(kLkThreads) k_ritz_k(const TQ* Q, const double* __restrict__ Z, int m, int k,
+                                                       int64_t n, TX* X) {
+  extern __shared__ double s_z[];
+  for (int t = threadIdx.x; t < m * K; t += blockDim.x) {
+    const int j = t / K, r = t - j * K;
+    s_z[t] = r < k ? Z[j + int64_t(r) * m] : 0.0;
+  }
+  __syncthreads();
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-    double acc[kMaxK];
+    double acc[K];
 #pragma unroll
-    for (int r = 0; r < kMaxK; ++r) acc[r] = 0.0;
+    for (int r = 0; r < K; ++r) acc[r] = 0.0;
+#pragma unroll 4
     for (int j = 0; j < m; ++j) {
       const double q = double(Q[int64_t(j) * n + i]);
 #pragma unroll
-      for (int r = 0; r < kMaxK; ++r)
-        if (r < k) acc[r] = __fma_rn(Z[j + int64_t(r) * m], q, acc[r]);
+      for (int r = 0; r < K; ++r) acc[r] = __fma_rn(s_z[j * K + r], q, acc[r]);
     }
 #pragma unroll
-    for (int r = 0; r < kMaxK; ++r)
-      if (r < k) X[int64_t(r) * n + i] = acc[r];
+    for (int r = 0; r < K; ++r)
+      if (r < k) X[int64_t(r) * n + i] = TX(acc[r]);
   }
+}
+
+// The k Ritz vectors in groups of at most 16 columns; in place (X == Q) all k at once, k <= 64.
+template <typename TQ, typename TX>
+int launch_ritz(const TQ* Q, const double* Z, int m, int k, int64_t n, TX* X, cudaStream_t st) {
+  const bool in_place = static_cast<const void*>(X) == static_cast<const void*>(Q);
+  if (in_place && k > 64) {
+    set_error("Ritz vectors in place: %d columns", k);
+    return EDG_ERR_ARG;
+  }
+  int64_t g = (n + kLkThreads - 1) / kLkThreads;
+  g = std::max<int64_t>(1, std::min<int64_t>(g, 148 * 8));
+  for (int r0 = 0; r0 < k; r0 += in_place ? k : 16) {
+    const int nr = in_place ? k : std::min(16, k - r0);
+    const int K = nr <= 4 ? 4 : nr <= 8 ? 8 : nr <= 16 ? 16 : nr <= 32 ? 32 : 64;
+    auto kern = K == 4    ? k_ritz_k<TQ, TX, 4>
+                : K == 8  ? k_ritz_k<TQ, TX, 8>
+                : K == 16 ? k_ritz_k<TQ, TX, 16>
+                : K == 32 ? k_ritz_k<TQ, TX, 32>
+                          : k_ritz_k<TQ, TX, 64>;
+    const size_t smem = size_t(m) * K * sizeof(double);
+    if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    kern<<<int(g), kLkThreads, smem, st>>>(Q, Z + size_t(r0) * m, m, nr, n, X + size_t(r0) * n);
+    EDG_CUDA(cudaGetLastError());
+  }
+  return EDG_OK;
 }
 
 // Dense sector matrix, column-major H[i + j*D] (W = 2: complex, interleaved, with the
@@ -527,7 +563,7 @@ struct LkRun {
     EDG_CHECK(coef.alloc(3 * size_t(ncv) + 8, st, "multi-dot coefficients"));
     EDG_CHECK(Gm.alloc(size_t(ncv) * ncv, st, "Gram matrix"));
     EDG_CHECK(dab.alloc(2 * size_t(ncv) + 4, st, "Lanczos scalars"));
-    DevBuf<double> Yc, Xr, Zd;
+    DevBuf<double> Yc, Zd;
     EDG_CHECK(Yc.alloc(size_t(ncv) * ncv, st, "projected matrix"));
     double* dA = dab.p;           // a_j of the current cycle (scratch)
     double* dB = dab.p + ncv + 1;  // b at column position t: dB[t]
@@ -639,20 +675,12 @@ struct LkRun {
         prev_lock = pl;
         next_check = steps + gap;
         if (full) {
-          // restart: X = Q Z[:, 0:pp] in FP64, then the first pp columns := X, column pp :=
-          // w / b, Gm := I on the leading pp + 1 columns, Hm := diag(theta) on them
+          // restart: the first pp columns := Q Z[:, 0:pp] (sums in FP64), column pp := w / b,
+          // Gm := I on the leading pp + 1 columns, Hm := diag(theta) on them
           const int pp = std::min(p, mm - 1);
-          EDG_CHECK(Xr.alloc(size_t(pp) * n, st, "thick-restart Ritz vectors"));
           EDG_CHECK(Zd.alloc(size_t(mm) * pp, st, "thick-restart coefficients"));
           EDG_CUDA(cudaMemcpyAsync(Zd.p, Zm.data(), size_t(mm) * pp * sizeof(double), cudaMemcpyHostToDevice, st));
-          for (int r0 = 0; r0 < pp; r0 += kMaxK) {
-            const int nr = std::min(kMaxK, pp - r0);
-            k_ritz_k<T><<<grid_n(n), kLkThreads, 0, st>>>(Q.p, Zd.p + size_t(r0) * mm, mm, nr, n,
-                                                          Xr.p + size_t(r0) * n);
-          }
-          EDG_CUDA(cudaGetLastError());
-          for (int r = 0; r < pp; ++r)
-            EDG_CHECK((convert_dev<T, double>(st, Q.p + size_t(r) * n, Xr.p + size_t(r) * n, n, 1.0)));
+          EDG_CHECK((launch_ritz<T, T>(Q.p, Zd.p, mm, pp, n, Q.p, st)));
           EDG_CHECK(scale_into<T>(st, Q.p + size_t(pp) * n, w.p, dB + mcur, n));
           k_gram_eye<<<((pp + 1) * (pp + 1) + 255) / 256, 256, 0, st>>>(Gm.p, ncv, pp + 1);
           EDG_CUDA(cudaGetLastError());
@@ -679,8 +707,7 @@ struct LkRun {
       DevBuf<double> Zd;
       EDG_CHECK(Zd.alloc(size_t(m) * kk, st, "Ritz coefficients"));
       EDG_CUDA(cudaMemcpyAsync(Zd.p, zf.data(), size_t(m) * kk * sizeof(double), cudaMemcpyHostToDevice, st));
-      k_ritz_k<T><<<grid_n(n), kLkThreads, 0, st>>>(Q.p, Zd.p, m, kk, n, X);
-      EDG_CUDA(cudaGetLastError());
+      EDG_CHECK((launch_ritz<T, double>(Q.p, Zd.p, m, kk, n, X, st)));
       EDG_CUDA(cudaStreamSynchronize(st));
     }
     return EDG_OK;
@@ -703,8 +730,7 @@ struct LkRun {
       DevBuf<double> Zd;
       EDG_CHECK(Zd.alloc(size_t(m) * kk, st, "Ritz coefficients"));
       EDG_CUDA(cudaMemcpyAsync(Zd.p, Z.data(), size_t(m) * kk * sizeof(double), cudaMemcpyHostToDevice, st));
-      k_ritz_k<T><<<grid_n(n), kLkThreads, 0, st>>>(Q.p, Zd.p, m, kk, n, X);
-      EDG_CUDA(cudaGetLastError());
+      EDG_CHECK((launch_ritz<T, double>(Q.p, Zd.p, m, kk, n, X, st)));
       EDG_CUDA(cudaStreamSynchronize(st));  // Z (host) is read by the copy above
     }
     return EDG_OK;
@@ -712,13 +738,11 @@ struct LkRun {
 };
 
 // Basis columns of precision `elem` that fit in HBM beyond a 2 GB reserve, at most mmax.
-// `kept`: FP64 vectors held next to the basis at a thick restart (0 without restarts).
-int basis_room(int64_t n, size_t elem, int k, int* mmax, int kept = 0) {
+int basis_room(int64_t n, size_t elem, int k, int* mmax) {
   size_t fr = 0, tot = 0;
   EDG_CUDA(cudaMemGetInfo(&fr, &tot));
   const size_t reserve = size_t(2) << 30, per = size_t(n) * elem;
-  // Ritz, start and restart vectors
-  const size_t extra = size_t(n) * sizeof(double) * (size_t(k) + 4 + size_t(kept));
+  const size_t extra = size_t(n) * sizeof(double) * (size_t(k) + 4);  // Ritz and start vectors
   const int64_t fit = fr > reserve + extra ? int64_t((fr - reserve - extra) / per) - 2 : 0;
   if (fit < *mmax) *mmax = int(fit);
   if (*mmax < k || *mmax < 1) {
@@ -768,7 +792,7 @@ int lowest_k(edg_sector_s* s, int k, const double* v0_host, uint64_t seed, int m
       EDG_CHECK(X.alloc(size_t(k) * n, st, "FP32 Ritz vectors"));
       {
         int nc = ncv;
-        EDG_CHECK(basis_room(n, sizeof(float), k, &nc, k + (nc - k) / 4));
+        EDG_CHECK(basis_room(n, sizeof(float), k, &nc));
         LkRun<float> r32;
         EDG_CHECK(r32.run_tr(s, k, x0.p, steps_max, nc, k + (nc - k) / 4, std::max(tol, kTol32)));
         steps32 = r32.steps;
@@ -779,7 +803,7 @@ int lowest_k(edg_sector_s* s, int k, const double* v0_host, uint64_t seed, int m
         for (int r = 0; r < k32; ++r) EDG_CHECK(axpy_accum_dev<double>(st, x0.p, X.p + size_t(r) * n, 1.0, n));
       }  // the FP32 basis goes back to the pool before the FP64 one is taken
     }
-    EDG_CHECK(basis_room(n, sizeof(double), k, &ncv, ncv < ne ? k + (ncv - k) / 4 : 0));
+    EDG_CHECK(basis_room(n, sizeof(double), k, &ncv));
     LkRun<double> r64;
     EDG_CHECK(r64.run_tr(s, k, x0.p, steps_max, ncv, k + (ncv - k) / 4, tol));
     if (niter) *niter = steps32 + r64.steps;
