@@ -531,8 +531,8 @@ static void build_schedule(int64_t dim, int rt, const std::vector<uint32_t>& off
 //  * any order: each lane takes a source from the free bank group with the most sources left;
 //    20.85 slots (an optimal edge colouring: 20.81).
 // width != null: counts the slots of each group only. Otherwise fills the entries of a slice
-// that starts at batch soff >> 9 and has (soff & 511) half batches of four slots; entries are
-// stored in batches of eight slots.
+// that starts at batch soff >> 9 and has (soff & 511) pairs of slots; entries are stored in
+// batches of eight slots.
 constexpr int kSchedMaxRow = 64;  // hops per column of the any-order schedule (a bit mask each)
 
 template <bool ORDERED>
@@ -566,7 +566,7 @@ __global__ void k_sched16(int64_t dim, const uint32_t* __restrict__ off, const u
   }
   const uint32_t so = width ? 0u : soff[oct / 4];
   const size_t base = size_t(so >> 9) * 256 + size_t(oct % 4) * G * 8;
-  const uint32_t slots = (so & 511u) * 4u;
+  const uint32_t slots = (so & 511u) * 2u;
   for (uint32_t c = 0; total || (!width && c < (slots + 7) / 8 * 8); ++c) {
     for (int i = 1; i < G; ++i)
       for (int j = i; j > 0 && left[ord[j]] > left[ord[j - 1]]; --j) {
@@ -691,10 +691,10 @@ int build_t16(edg_sector_s* s, const BondList& bl, SpinBasis& B) {
     for (int64_t sl = 0; sl < nsl; ++sl) {
       uint32_t m = 1;
       for (int g = 0; g < 4; ++g) m = std::max(m, w[o * noct + sl * 4 + g]);
-      const uint32_t half = (m + 3) / 4;
-      if (half > 511 || nb >= (1u << 23)) return EDG_OK;
-      soff[o * nsl + sl] = nb << 9 | half;
-      nb += (half + 1) / 2;
+      const uint32_t pairs = (m + 1) / 2;
+      if (pairs > 511 || nb >= (1u << 23)) return EDG_OK;
+      soff[o * nsl + sl] = nb << 9 | pairs;
+      nb += (pairs + 3) / 4;
     }
     EDG_CHECK(B.t16_off[o].alloc(nsl, st, "slot schedule"));
     EDG_CHECK(B.t16_ent[o].alloc(size_t(nb) * 256, st, "slot schedule"));

@@ -170,7 +170,7 @@ struct SpinBasis {
   // (FP32, uniform tables). Entry: bits 0..14 the shared-memory slot of the source (DimUp +
   // 0..7: a zero slot), bit 15 the sign of the uniform value. A batch is eight slots, lane l's
   // eight entries side by side (one 16-byte load); t16_off holds each slice's first
-  // batch << 9 | its half batches. Tables of more than one |value| keep a
+  // batch << 9 | its pairs of slots. Tables of more than one |value| keep a
   // palette of at most 256 values instead of the sign, one 8-bit code per entry.
   bool t16 = false;
   DevBuf<uint16_t> t16_ent[2];

@@ -19,10 +19,12 @@
 // takes 4 wavefronts (one per 8 lanes) and half a wavefront of entries; in source order without
 // a schedule bank conflicts took 36-39 wavefronts per 8 lanes and 16-17 hops on the 4x4
 // lattice, with it 22-23. Where a tile fills an SM, staging it is next (a fifth of the pass
-// from HBM; the next tile's rows are therefore fetched into L2 ahead).
+// from HBM; the next tile's rows are therefore fetched into L2 ahead). A slice ends at a pair of
+// slots: ending at four cost 5 % more slots (24.0 against 22.9 on that lattice, any order) and
+// 1-3 % of the product.
 // Measured, before (32-bit SELL entries, two FP32 or two FP64 rows) and now, us:
-//   up pass, 4x4 (8,8)  FP32  1025 -> 817     4x4 (7,7) FP64  1862 -> 1294
-//   up pass, 5x3 (7,8)  FP64   570 -> 398     fused Lanczos 4x4 (6,6) FP64  1084 -> 804
+//   up pass, 4x4 (8,8)  FP32  1025 -> 808     4x4 (7,7) FP64  1862 -> 1294
+//   up pass, 5x3 (7,8)  FP64   570 -> 397     fused Lanczos 4x4 (6,6) FP64  1084 -> 804
 //   whole product, 3x4 (6,6) FP64: two passes 44.0 -> 22.3; 12 Lanczos columns 491 -> 202
 //   complex128 4x4 (5,5): 2433 (one thread per element, L1 gathers) -> 1157 in two passes;
 //   3x4 (6,6) 81 -> 44, 4x4 (4,5) 825 -> 326 in one launch
@@ -39,7 +41,7 @@ template <typename T, int W>
 struct TileArgs {
   const uint4* __restrict__ ent;       // eight 16-bit entries per lane and batch
   const uint2* __restrict__ code;      // eight palette codes per lane and batch (PAL)
-  const uint32_t* __restrict__ off;    // [nsl] first batch of a slice << 9 | its half batches (four slots)
+  const uint32_t* __restrict__ off;    // [nsl] first batch of a slice << 9 | its slot pairs
   const double* __restrict__ pal;      // palette: W doubles per code (PAL)
   T h;                                 // value of sign bit 0 (!PAL)
   T h_dw = T(0);                       // the same of the down hops
@@ -178,7 +180,8 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
     // The first entries, (rows-in form) sums and (down form) diagonal terms of each slice are
     // loaded while the slice before it runs, the first one's while the tile is staged.
     int sl = s0 + warp;
-    uint32_t o = 0, o1 = 0;
+    uint32_t o = 0;  // next batch
+    int np = 0;      // slot pairs left
     uint4 b0 = make_uint4(0u, 0u, 0u, 0u);
     uint2 c0 = make_uint2(0u, 0u);
     E hn[RT] = {};
@@ -186,10 +189,10 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
     uint32_t mun = 0;
     if (sl < s1) {
       const uint32_t w = q.off[sl];
-      o = (w >> 9) * 2;
-      o1 = o + (w & 511u);
-      b0 = __ldg(q.ent + o * 16u + lane);
-      if (PAL) c0 = __ldg(q.code + o * 16u + lane);
+      o = w >> 9;
+      np = int(w & 511u);
+      b0 = __ldg(q.ent + o * 32u + lane);
+      if (PAL) c0 = __ldg(q.code + o * 32u + lane);
       const int c = min(sl * 32 + lane, dimup - 1);
       if (DIAG) {
         eun = a.e_up[c];
@@ -241,11 +244,12 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
       const int nsl = sl + nw;
       const bool more = nsl < s1;
       const int cn = min(nsl * 32 + lane, dimup - 1);
-      uint32_t on = o, on1 = o1;
+      uint32_t on = o;
+      int npn = np;
       if (more) {
         const uint32_t w = s_off[nsl];
-        on = (w >> 9) * 2;
-        on1 = on + (w & 511u);
+        on = w >> 9;
+        npn = int(w & 511u);
       }
       if (!DOWN) {
         // The next tile's rows into L2 during the second half of this one: with one CTA per SM
@@ -364,30 +368,37 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
       }
       SlotAcc<T, W> acc;
       acc.set(acc0);
-      for (uint32_t p = o; p < o1; p += 2) {
+      // one slot: bits 0..14 its 16 bytes, bit 15 the sign
+      auto slot = [&](uint32_t ww, bool odd, uint32_t cd) {
+        const uint32_t at = sbase + (odd ? (ww >> 12) & 0x7fff0u : (ww << 4) & 0x7fff0u);
+        ulonglong2 x;
+        asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(x.x), "=l"(x.y) : "r"(at));
+        T h[W];
+        if (PAL) {
+          const T* pv = s_pal + (cd & 0xffu) * W;
+#pragma unroll
+          for (int w = 0; w < W; ++w) h[w] = pv[w];
+        } else {
+          h[0] = flip_sign(hs, odd ? ww : ww << 16);
+        }
+        acc.fma(h, x);
+      };
+      for (; np > 0; np -= 4) {
         const uint4 wq = b0;
         const uint2 cq = c0;
-        const uint32_t nx = (p + 2 < o1 ? p + 2 : on) * 16u + lane;
+        const uint32_t nx = (np > 4 ? ++o : on) * 32u + lane;
         b0 = __ldg(q.ent + nx);
         if (PAL) c0 = __ldg(q.code + nx);
         const uint32_t ws[4] = {wq.x, wq.y, wq.z, wq.w};
+        if (np >= 4) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          if (u == 4 && p + 1 == o1) break;  // an odd number of half batches
-          const uint32_t ww = ws[u >> 1];
-          // bits 0..14 slot, bit 15 sign
-          const uint32_t at = sbase + ((u & 1) ? (ww >> 12) & 0x7fff0u : (ww << 4) & 0x7fff0u);
-          ulonglong2 x;
-          asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(x.x), "=l"(x.y) : "r"(at));
-          T h[W];
-          if (PAL) {
-            const T* pv = s_pal + (((u < 4 ? cq.x : cq.y) >> (8 * (u & 3))) & 0xffu) * W;
+          for (int u = 0; u < 8; ++u) slot(ws[u >> 1], u & 1, (u < 4 ? cq.x : cq.y) >> (8 * (u & 3)));
+        } else {  // the slice's last pairs
 #pragma unroll
-            for (int w = 0; w < W; ++w) h[w] = pv[w];
-          } else {
-            h[0] = flip_sign(hs, (u & 1) ? ww : ww << 16);
+          for (int u = 0; u < 6; ++u) {
+            if (u >= 2 * np) break;
+            slot(ws[u >> 1], u & 1, (u < 4 ? cq.x : cq.y) >> (8 * (u & 3)));
           }
-          acc.fma(h, x);
         }
       }
       if (SUB && !DOWN) {
@@ -430,7 +441,7 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
       }
       sl = nsl;
       o = on;
-      o1 = on1;
+      np = npn;
     }
     __syncthreads();
   }
