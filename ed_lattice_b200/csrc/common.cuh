@@ -482,7 +482,7 @@ int sector_dense_dev(edg_sector_s* s, double* dH);
 int tridiag_eigh_host(int n, const double* d, const double* e, double* w, double* z1, double* zfull,
                       double* zn = nullptr);
 // k lowest eigenvalues and |last eigenvector components| (bisection + twisted factorisation)
-int tridiag_lowest_host(int n, const double* d, const double* e, int k, double* w, double* zn);
+int tridiag_lowest_host(int n, const double* d, const double* e, int k, double* w, double* zn, int kz = 1 << 30);
 // k lowest eigenpairs (vectors z[k][n]) by bisection + twisted factorisation; EDG_ERR_NOCONV
 // when two of the k+1 lowest eigenvalues are closer than relgap * spectral radius
 int tridiag_lowest_vectors(int n, const double* d, const double* e, int k, double relgap, double* w, double* z);

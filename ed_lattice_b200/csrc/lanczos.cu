@@ -20,6 +20,7 @@
 // the host once per step (16 bytes) for the convergence test.
 #include <algorithm>
 #include <cmath>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -128,24 +129,25 @@ struct Recurrence {
   }
   // device array of b_{j+1} (index j+1)
   const double* b_dev() const { return fused ? sc.bn : sc.b; }
-  // step j: W <- the unnormalised u_{j+1}; returns a_j and b_{j+1} on the host
-  int step(int j, double* a, double* b) {
-    EDG_CHECK(step_dev(j));
-    return read(j, a, b);
-  }
-  // a_j and b_{j+1} of a queued step j, on the host (waits for step j)
-  int read(int j, double* a, double* b) {
-    cudaStream_t st = s->stream;
-    double h[2];
-    EDG_CUDA(cudaMemcpyAsync(&h[0], sc.a + j, sizeof(double), cudaMemcpyDeviceToHost, st));
-    EDG_CUDA(cudaMemcpyAsync(&h[1], (fused ? sc.bn : sc.b) + j + 1, sizeof(double), cudaMemcpyDeviceToHost, st));
-    EDG_CUDA(cudaStreamSynchronize(st));
-    *a = h[0];
-    *b = h[1];
+  // a_j and b_{j+1} of the queued step j into ab[2], in stream order; `done` fires when they are there
+  int post(int j, double* ab, cudaEvent_t done) {
+    const double* b = b_dev() + j + 1;
+    EDG_CUDA(cudaMemcpy2DAsync(ab, sizeof(double), sc.a + j, size_t(b - (sc.a + j)) * sizeof(double), sizeof(double), 2,
+                               cudaMemcpyDeviceToHost, s->stream));
+    EDG_CUDA(cudaEventRecord(done, s->stream));
     return EDG_OK;
   }
   // after step j with b = b_{j+1} > 0: make U hold (a multiple of) v_{j+1}
   int advance(int j, double b) {
+    EDG_CHECK(advance_dev(j));
+    norm(b);
+    return EDG_OK;
+  }
+  // the norm of the vector that advance_dev made current, once the host knows it
+  void norm(double b) {
+    if (fused) bn_host.push_back(b);
+  }
+  int advance_dev(int j) {
     if (fused) {
       T* t = P;
       P = U;
@@ -157,7 +159,6 @@ struct Recurrence {
       } else {
         W = t;
       }
-      bn_host.push_back(b);
     } else {
       EDG_CHECK(scale_into<T>(s->stream, P, W, sc.b + j + 1, s->vlen));
       T* t = P;
@@ -335,6 +336,74 @@ Ritz lowest_ritz(const std::vector<double>& a, const std::vector<double>& b, dou
   return r;
 }
 
+// The same from bisection and one twisted factorisation, O(m): e0 to a few ulps of the spectral
+// radius, err to a few per cent. False where it might not be: a short chain, two Ritz values
+// within rounding of each other, or more copies than one bisection covers.
+// 100 steps, host: 0.3 ms with the QL iteration above, 0.06 here.
+bool estimate_ritz(const std::vector<double>& a, const std::vector<double>& b, double b_next, double window, Ritz* r) {
+  constexpr int kLow = 8;  // Ritz values bisected together
+  const int m = int(a.size());
+  if (m <= 2 * kLow) return false;
+  double w[kLow], z;
+  if (tridiag_lowest_host(m, a.data(), b.data(), kLow, w, &z, 1) != EDG_OK) return false;
+  if (w[1] - w[0] <= 1e-12 * std::fabs(w[0])) return false;
+  int i = 1;
+  while (i < kLow && w[i] - w[0] <= window * std::fabs(w[0])) ++i;
+  if (i == kLow) return false;
+  const double res = b_next * z, gap = w[i] - w[0];
+  r->e0 = w[0];
+  r->err = gap > 1e-12 ? res * res / gap : res;
+  return true;
+}
+
+// 16 bytes of page-locked host memory, where a step's coefficients land while later steps are
+// queued. The slots of one 4 KB page of the process, taken by one run at a time and given back
+// with it; without a free one the copy goes to pageable memory and waits for the step.
+class HostPair {
+ public:
+  HostPair() {
+    std::lock_guard<std::mutex> lock(mu());
+    double*& page = base();
+    if (!page) {
+      // an allocation may not disturb a capture that another thread has open
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      void* q = nullptr;
+      if (cudaHostAlloc(&q, kSlots * 64, cudaHostAllocPortable) == cudaSuccess) page = static_cast<double*>(q);
+      else (void)cudaGetLastError();
+      cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    for (int i = 0; page && i < kSlots && slot_ < 0; ++i)
+      if (!(used() >> i & 1)) slot_ = i;
+    if (slot_ >= 0) {
+      used() |= uint64_t(1) << slot_;
+      p = page + slot_ * 8;
+    }
+  }
+  ~HostPair() {
+    std::lock_guard<std::mutex> lock(mu());
+    if (slot_ >= 0) used() &= ~(uint64_t(1) << slot_);
+  }
+  HostPair(const HostPair&) = delete;
+  HostPair& operator=(const HostPair&) = delete;
+  double* p = own_;
+
+ private:
+  static constexpr int kSlots = 64;  // a cache line each
+  static std::mutex& mu() { static std::mutex m; return m; }
+  static double*& base() { static double* b = nullptr; return b; }
+  static uint64_t& used() { static uint64_t u = 0; return u; }
+  double own_[2] = {0.0, 0.0};
+  int slot_ = -1;
+};
+
+struct Event {
+  cudaEvent_t e = nullptr;
+  ~Event() {
+    if (e) cudaEventDestroy(e);
+  }
+};
+
 // Plain Lanczos in precision T from the normalised FP64 device vector dv0 until the lowest
 // Ritz value is converged to tol (see lowest_ritz), b underflows, or maxit. Optionally stores
 // the normalised basis vectors in FP32 so the Ritz vector needs no second pass.
@@ -349,55 +418,76 @@ int gs_run(edg_sector_s* s, const double* dv0, int maxit, double tol, std::vecto
   A->clear();
   B->assign(1, 0.0);
   colscale->clear();
-  // the basis column of step j (before the step is queued)
+  // the basis column of step j (before the step is queued); the fused form writes it in place
   auto column = [&](int j) -> int {
-    if (basis && j < basis_cols) {
-      if (R.ext) {
-        colscale->push_back(R.vscale(j));  // column j holds u_j = v_j / vscale(j)
-      } else {
-        EDG_CHECK((convert_dev<float, T>(st, basis + size_t(j) * n, R.U, n, R.vscale(j))));
-        colscale->push_back(1.0);
-      }
-    }
+    if (basis && j < basis_cols && !R.ext)
+      EDG_CHECK((convert_dev<float, T>(st, basis + size_t(j) * n, R.U, n, R.vscale(j))));
     return EDG_OK;
   };
+  HostPair ab;
+  Event done;
+  EDG_CUDA(cudaEventCreateWithFlags(&done.e, cudaEventDisableTiming));
+  // FP32 vectors lose orthogonality within tens of steps: skip the copies of E0 that follow
+  const double window = sizeof(T) == 4 ? 10.0 * tol : 0.0;
   double eold = 0.0, err_prev = HUGE_VAL;
+  bool eold_exact = true;
   bool queued = false;  // step j was queued by the previous iteration
   for (int j = 0; j < maxit; ++j) {
     if (!queued) {
       EDG_CHECK(column(j));
       EDG_CHECK(R.step_dev(j));
     }
-    double a, b;
-    EDG_CHECK(R.read(j, &a, &b));
-    if (!std::isfinite(a) || !std::isfinite(b)) {
-      set_error("Lanczos produced a non-finite coefficient at step %d", j);
-      return EDG_ERR_NOCONV;
-    }
-    A->push_back(a);
+    EDG_CHECK(R.post(j, ab.p, done.e));
     // While the last test was far from convergence (its error estimate more than 100x the
-    // target 0.1 tol |E0|), step j+1 is queued before step j is tested, so the host's test
-    // runs while the GPU works; near convergence the test comes first, so no step is wasted.
-    queued = j + 1 < maxit && b >= 1e-14 && err_prev > 10.0 * tol * std::fabs(eold);
+    // target 0.1 tol |E0|), step j+1 is queued before the host waits for step j, so the GPU
+    // goes from step to step; near convergence the test comes first, so no step is wasted.
+    // Per call, U = 8, FP64, the wait first and a QL iteration every step -> this: 245,025
+    // states 20.7 -> 7.9 ms, 853,776 18.4 -> 8.5, 9.0 M 53.9 -> 40.3, 64 M 249 -> 245.
+    queued = j + 1 < maxit && err_prev > 10.0 * tol * std::fabs(eold);
     if (queued) {
-      EDG_CHECK(R.advance(j, b));
+      EDG_CHECK(R.advance_dev(j));
       EDG_CHECK(column(j + 1));
       EDG_CHECK(R.step_dev(j + 1));
     }
-    // FP32 vectors lose orthogonality within tens of steps: skip the copies of E0 that follow
-    const Ritz rz = lowest_ritz(*A, *B, b, sizeof(T) == 4 ? 10.0 * tol : 0.0);
-    const double e = rz.e0;
+    EDG_CUDA(cudaEventSynchronize(done.e));
+    const double a = ab.p[0], b = ab.p[1];
+    if (!std::isfinite(a) || !std::isfinite(b)) {
+      (void)cudaStreamSynchronize(st);
+      set_error("Lanczos produced a non-finite coefficient at step %d", j);
+      return EDG_ERR_NOCONV;
+    }
+    // column j holds u_j = v_j / vscale(j) when written in place
+    if (basis && j < basis_cols) colscale->push_back(R.ext ? R.vscale(j) : 1.0);
+    A->push_back(a);
     // converged when the error estimate is 10x below tol*|E0| (or, as a fallback for a
     // degenerate lowest level, when E0 stops moving), or the Krylov space is exhausted; a
     // step queued ahead is then discarded (its column lies past the Ritz vector's)
-    const bool conv = (j > 0 && rz.err <= 0.1 * tol * std::fabs(e)) ||
-                      (j > 0 && std::fabs(e - eold) <= 0.01 * tol * std::fabs(e)) || b < 1e-14;
-    eold = e;
+    auto settled = [&](const Ritz& r, double slack, double noise) {
+      return b < 1e-14 || (j > 0 && (r.err <= slack * 0.1 * tol * std::fabs(r.e0) ||
+                                     std::fabs(r.e0 - eold) <= slack * 0.01 * tol * std::fabs(r.e0) + noise));
+    };
+    // The QL iteration decides, and gives E0; it is left out where the estimate is four times
+    // (and, for the change of E0, the rounding of two bisections) away from either limit.
+    Ritz rz;
+    bool exact = j + 1 == maxit || !estimate_ritz(*A, *B, b, window, &rz);
+    if (!exact) exact = settled(rz, 4.0, 1e-13 * (std::fabs(rz.e0) + b));
+    bool conv = false;
+    if (exact) {
+      if (!eold_exact) {
+        const std::vector<double> before(A->begin(), A->end() - 1);
+        eold = lowest_ritz(before, *B, 0.0, window).e0;
+      }
+      rz = lowest_ritz(*A, *B, b, window);
+      conv = settled(rz, 1.0, 0.0);
+    }
+    eold = rz.e0;
+    eold_exact = exact;
     err_prev = rz.err;
     B->push_back(b);
-    *e0 = e;
+    *e0 = rz.e0;
     if (conv || j + 1 == maxit) break;
-    if (!queued) EDG_CHECK(R.advance(j, b));
+    if (!queued) EDG_CHECK(R.advance_dev(j));
+    R.norm(b);
   }
   EDG_CUDA(cudaStreamSynchronize(st));  // a discarded step still runs on the work vectors
   return EDG_OK;
@@ -429,9 +519,8 @@ int ritz_vector(edg_sector_s* s, const double* dv0, const std::vector<double>& A
     for (int j = 0; j < m; ++j) {
       EDG_CHECK(axpy_accum_dev<T>(st, x, R.U, Z[j] * R.vscale(j), n));
       if (j + 1 == m) break;
-      double a, b;
-      EDG_CHECK(R.step(j, &a, &b));
-      EDG_CHECK(R.advance(j, b));
+      EDG_CHECK(R.step_dev(j));
+      EDG_CHECK(R.advance(j, B[j + 1]));  // the steps repeat the run's own, bit for bit
     }
   }
   // normalise

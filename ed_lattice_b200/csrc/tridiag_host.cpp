@@ -226,9 +226,9 @@ void bisect_lowest(int n, const double* d, const double* e, int k, double* w, st
 
 }  // namespace
 
-// k lowest eigenvalues ascending and |last component| of each unit eigenvector, O(k n);
+// k lowest eigenvalues ascending and |last component| of the first kz unit eigenvectors, O(k n);
 // used to test Lanczos convergence on the k lowest Ritz pairs between steps.
-int tridiag_lowest_host(int n, const double* d, const double* e, int k, double* w, double* zn) {
+int tridiag_lowest_host(int n, const double* d, const double* e, int k, double* w, double* zn, int kz) {
   if (n <= 0 || k <= 0) return EDG_OK;
   if (k > n) k = n;
   std::vector<double> e2;
@@ -236,7 +236,7 @@ int tridiag_lowest_host(int n, const double* d, const double* e, int k, double* 
   bisect_lowest(n, d, e, k, w, e2, &pivmin, &span);
   if (!zn) return EDG_OK;
   std::vector<double> dp(n), rm(n), z(n);
-  for (int j = 0; j < k; ++j) {
+  for (int j = 0; j < std::min(k, kz); ++j) {
     EDG_CHECK(twisted_vector(n, d, e, e2.data(), w[j], pivmin, dp.data(), rm.data(), z.data()));
     zn[j] = std::fabs(z[n - 1]);
   }
