@@ -25,7 +25,7 @@
 // Measured, before (32-bit SELL entries, two FP32 or two FP64 rows) and now, us:
 //   up pass, 4x4 (8,8)  FP32  1025 -> 808     4x4 (7,7) FP64  1862 -> 1294
 //   up pass, 5x3 (7,8)  FP64   570 -> 397     fused Lanczos 4x4 (6,6) FP64  1084 -> 804
-//   whole product, 3x4 (6,6) FP64: two passes 44.0 -> 22.3; 12 Lanczos columns 491 -> 202
+//   whole product, 3x4 (6,6) FP64: two passes 44.0 -> 22.3; 12 Lanczos columns 491 -> 187
 //   complex128 4x4 (5,5): 2433 (one thread per element, L1 gathers) -> 1157 in two passes;
 //   3x4 (6,6) 81 -> 44, 4x4 (4,5) 825 -> 326 in one launch
 #include <algorithm>
@@ -45,6 +45,7 @@ struct TileArgs {
   const double* __restrict__ pal;      // palette: W doubles per code (PAL)
   T h;                                 // value of sign bit 0 (!PAL)
   T h_dw = T(0);                       // the same of the down hops
+  bool two = false;                    // each warp stands for two of the sum <v, w>
   int npal = 0;
   int nsl = 0, ntile = 0;
   int csplit = 1;                      // column parts of a tile, each its own work item
@@ -154,7 +155,8 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
   __shared__ uint32_t s_mdw[RT];
   __shared__ int s_cnt[RT];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  double pa = 0.0, sc = 1.0;
+  // <v, w>: slices 0, nw, 2 nw, ... of the warp, or (q.two) every other one of them into each
+  double pa[2] = {0.0, 0.0}, sc = 1.0;
   if (LZ) {
     sc = 1.0 / a.bn[a.jstep];
     if (threadIdx.x == 0) {
@@ -180,6 +182,7 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
     // The first entries, (rows-in form) sums and (down form) diagonal terms of each slice are
     // loaded while the slice before it runs, the first one's while the tile is staged.
     int sl = s0 + warp;
+    bool odd = false;
     uint32_t o = 0;  // next batch
     int np = 0;      // slot pairs left
     uint4 b0 = make_uint4(0u, 0u, 0u, 0u);
@@ -415,15 +418,19 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
         const double scl = s_lz[0], cc = s_lz[1];
         const ulonglong2 xc = S[c];
         const T* xs = reinterpret_cast<const T*>(&xc);
+        double p1 = DOWN && odd ? pa[1] : pa[0];
 #pragma unroll
         for (int r = 0; r < RT; ++r)
           if (act && r < rows) {
             const T wt = SUB ? T(double(res[r]) - cc * double(up[r])) : res[r];
-            pa = __fma_rn(double(xs[r]) * scl, double(wt), pa);
+            p1 = __fma_rn(double(xs[r]) * scl, double(wt), p1);
             T* p = a.hv + (r0 + r) * dimup + c;
             if (DOWN) *p = wt;
             else __stcs(p, wt);
           }
+        if (DOWN && odd) pa[1] = p1;
+        else pa[0] = p1;
+        if (DOWN) odd = q.two && !odd;
       } else {
 #pragma unroll
         for (int r = 0; r < RT; ++r)
@@ -447,12 +454,17 @@ __global__ void __launch_bounds__(1024, 1) k_tile(HxvArgs<T> a, TileArgs<T, W> q
   }
   if (LZ) {  // block partial of <v, w>, fixed order
     __shared__ double s_red[32];
-    for (int d = 16; d > 0; d >>= 1) pa += __shfl_down_sync(0xffffffffu, pa, d);
-    if (lane == 0) s_red[warp] = pa;
+    const int ng = DOWN && q.two ? 2 * nw : nw;
+#pragma unroll
+    for (int g = 0; g < (DOWN ? 2 : 1); ++g) {
+      if (g * nw >= ng) break;
+      for (int d = 16; d > 0; d >>= 1) pa[g] += __shfl_down_sync(0xffffffffu, pa[g], d);
+      if (lane == 0) s_red[warp + g * nw] = pa[g];
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
       double t = 0.0;
-      for (int w = 0; w < nw; ++w) t += s_red[w];
+      for (int w = 0; w < ng; ++w) t += s_red[w];
       a.partial[blockIdx.x] = t;
     }
     finish_in_last_block(a.partial, gridDim.x, a.red_out, 0);
@@ -483,7 +495,16 @@ int launch(const HxvArgs<T>& a, TileArgs<T, W>& q, cudaStream_t st, int sms) {
     else
       q.csplit = std::max(1, std::min((3 * sms * per_sm / 4 + q.ntile - 1) / q.ntile, q.nsl / warps));
     const int most = (q.nsl + q.csplit - 1) / q.csplit, rounds = (most + warps - 1) / warps;
-    warps = (most + rounds - 1) / rounds;
+    // Two waves or more of CTAs of four warps, eight per SM: their staging and their last rounds
+    // overlap better than those of four CTAs of eight (12 Lanczos columns, FP64: 731,808 states
+    // 208 -> 187 us, 4x3 (4,4) 133 -> 115; 4x4 (3,8) 147 -> 134; with fewer tiles, 7x2 (4,7),
+    // 51 -> 57). The sum <v, w> is the one that eight warps form, so it does not change with the
+    // number of columns.
+    const bool small = per_sm == 4 && most > 4 && 8 * (smem + 2048) <= 227 * 1024 &&
+                       int64_t(q.ntile) * q.csplit * a.ncols >= int64_t(sms) * 16;
+    if (small) warps = 4;
+    else if (!LZ || per_sm < 4 || most <= warps) warps = (most + rounds - 1) / rounds;
+    q.two = small;
   }
   const int threads = 32 * warps;
   int64_t g = int64_t(q.ntile) * q.csplit;

@@ -160,3 +160,27 @@ def test_hxv_tile_complex(case, prec, form):
     d = np.abs(y.cpu().numpy() - ref).max() / np.abs(ref).max()
     assert d <= (1e-13 if prec == "f64" else 2e-6), d
     s.delete()
+
+
+@pytest.mark.parametrize("case", [(10, 1, 5, 5, 20, "f64"),  # 252 columns: one slice per warp against two
+                                  (3, 4, 4, 4, 12, "f64"), (3, 4, 5, 6, 12, "f32"), (4, 4, 3, 4, 3, "f64"),
+                                  (7, 2, 4, 7, 2, "f64")], ids=lambda c: "%dx%d_%d_%d_x%d_%s" % c)
+def test_many_columns_are_single_chains(case):
+    """Blocks whose tiles go to CTAs of four warps: the coefficients of each column are those of
+    a chain of its own, whose CTAs have eight, bit for bit."""
+    import torch
+    lx, ly, nup, ndw, k, prec = case
+    p = E.EDG_PREC_F64 if prec == "f64" else E.EDG_PREC_F32
+    s = E.Sector(E.Model(lattice(lx, ly), uloc=4.0, xmu=2.0, hfmode=False), nup, ndw)
+    X = torch.tensor(np.stack([O.random_vector(50 + c, s.dim) for c in range(k)]), dtype=torch.float64, device="cuda")
+    n, pd, pi = 20, L._pd, L._pi
+    a, b, n2, ns = np.zeros((k, n)), np.zeros((k, n)), np.zeros(k), np.zeros(k, dtype=np.int32)
+    L.check(L.lib().edg_tridiag_block_dev(s.handle, k, C.c_void_p(X.data_ptr()), n, 1e-9, p, a.ctypes.data_as(pd),
+                                          b.ctypes.data_as(pd), n2.ctypes.data_as(pd), ns.ctypes.data_as(pi)), "block")
+    for c in (0, k // 2, k - 1):
+        a1, b1, n21, ns1 = np.zeros(n), np.zeros(n), C.c_double(), C.c_int()
+        L.check(L.lib().edg_tridiag_dev_f64(s.handle, C.c_void_p(X[c].data_ptr()), n, 1e-9, p, a1.ctypes.data_as(pd),
+                                            b1.ctypes.data_as(pd), C.byref(n21), C.byref(ns1)), "single")
+        assert ns[c] == ns1.value == n and n2[c] == n21.value
+        assert np.array_equal(a[c], a1) and np.array_equal(b[c], b1), c
+    s.delete()
