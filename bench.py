@@ -38,7 +38,7 @@ METRIC = "hxv_algorithmic_GBps"
 UNIT = "GB/s"
 # DRAM read + write of the kernels of one FP32 H x v of this sector (dram__bytes_read.sum +
 # dram__bytes_write.sum over the launches of one H x v), a constant taken from an ncu capture
-TRAFFIC_GB = 3.233
+TRAFFIC_GB = 3.238
 TRAFFIC_SOURCE = "ncu, constant from a capture of the same H x v (not measured in this run)"
 
 
@@ -595,9 +595,9 @@ def run_ours(args):
                          "traffic": TRAFFIC_GB, "traffic_unit": "GB per H x v",
                          "traffic_source": TRAFFIC_SOURCE},
             "clocks": clk.summary(),
-            "autotune": {"candidates": "3*down + up; down: 0 row groups, 1 block-staged 1 CTA/SM, 2 block-staged "
-                                       "2 CTAs/SM; up (FP32): 0 SELL-32, 1 packed 16-bit negated copies, 2 packed "
-                                       "16-bit sign bits", **tune},
+            "autotune": {"candidates": "4*down + up; down: 0 row groups, 1 block-staged 1 CTA/SM, 2 block-staged "
+                                       "2 CTAs/SM, 3 single pass (no up); up (FP32): 0 row tiles, 1 packed 16-bit "
+                                       "negated copies, 2 packed 16-bit sign bits, 3 Kronecker", **tune},
             "gpu_launches": 2 * args.steps,
             "e2e": e2e,
             "cpu_baseline": cpu,
