@@ -397,10 +397,13 @@ class HostPair {
   int slot_ = -1;
 };
 
+// Waits, on every way out, for the copy that it was last recorded after: the slot is free then.
 struct Event {
   cudaEvent_t e = nullptr;
   ~Event() {
-    if (e) cudaEventDestroy(e);
+    if (!e) return;
+    (void)cudaEventSynchronize(e);
+    (void)cudaEventDestroy(e);
   }
 };
 
