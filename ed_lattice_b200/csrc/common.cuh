@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/edgpu.h"
+#include "limits.h"
 
 namespace edg {
 
@@ -334,14 +335,6 @@ namespace edg {
 constexpr size_t kUpSmemTwoPerSM = 113 * 1024;
 constexpr size_t kUpSmemOnePerSM = 227 * 1024;
 constexpr int kUpZeroSlots = 32;
-constexpr int kT16Zero = 8;    // zero slots after a tile, one per 16-byte bank group
-// Shared memory of a tile kernel: the slots, `hops` down hops (value and source row) and the
-// palette of `elem`-byte values, the slices' offsets.
-constexpr size_t kTileSmemMax = 226 * 1024;  // leaves room for the kernels' static arrays
-inline size_t tile_smem(int64_t dimup, int npal, int hops, size_t elem) {
-  return size_t(dimup + kT16Zero) * 16 + size_t(hops) * ((elem + sizeof(uint32_t) + 7) / 8 * 8) + size_t(npal) * elem +
-         size_t((dimup + 31) / 32) * sizeof(uint32_t);
-}
 constexpr int kSellBatch = 8;  // SELL slice widths are multiples of this (entries loaded per batch)
 inline int up_rows_per_cta(int64_t dimup, size_t elem) {
   const size_t row = size_t(dimup + kUpZeroSlots) * elem;

@@ -1608,7 +1608,8 @@ HxvArgs<T> make_args(edg_sector_s* s, const T* v, T* hv) {
 }
 
 // Single-pass H x v (down-pass choice 3): one launch does the whole H x v; no up pass.
-// By row tiles (tile.cu) where the tile kernels apply, else the per-column gathers.
+// By row tiles (tile.cu) where the tile kernels apply, else the per-column gathers, which index
+// in 64 bits: edg_sector_set_kernels and edg_sector_autotune choose this pass for any size.
 template <typename T, bool LZ>
 int fused_pass(edg_sector_s* s, const HxvArgs<T>& a, cudaStream_t st, int sms) {
   if (tile_available(s, sizeof(T), true) && s->dim >= (sizeof(T) == 8 ? kTileMinDim64 : kTileMinDim32))

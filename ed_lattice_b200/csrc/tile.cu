@@ -553,7 +553,7 @@ int tile_pass(const HxvArgs<T>& a, const SpinBasis& up, const SpinBasis& dw, con
 
 bool tile_available(const edg_sector_s* s, size_t elem, bool down) {
   const SpinBasis& up = s->up;
-  if (!up.t16) return false;
+  if (!up.t16 || (down && !tile_down_index(s->dim))) return false;
   const int rt = int(16 / elem);  // elem: bytes per vector element (a complex one counts whole)
   // the single-value form of the whole product needs one |value| on either side
   if (down && up.t16_npal == 0 && !s->dw.sell_uniform) return false;
