@@ -362,6 +362,11 @@ int build_tables(edg_sector_s* s, int spin, SpinBasis& B) {
   cudaStream_t st = s->stream;
   const BondList& bl = s->bonds[spin - 1];
   const int nb = bl.nb;
+  const uint64_t total = hop_total(s->model.ns, B.nel, nb);
+  if (!table_fits(total)) {
+    set_error("hop table of spin %d: %llu hops, offsets are 32-bit", spin, (unsigned long long)total);
+    return EDG_ERR_UNSUPPORTED;
+  }
   DevBuf<int32_t> bonds;
   DevBuf<double> bh, bhi;
   std::vector<int32_t> hb(2 * nb + 2);
@@ -1098,6 +1103,9 @@ int build_variants(edg_sector_s* s, SpinBasis& B) {
 int build_sell(edg_sector_s* s, SpinBasis& B, bool up) {
   cudaStream_t st = s->stream;
   const int64_t dim = B.dim;
+  // complex and direct sectors read all of this with the tile kernels alone
+  if ((s->cplx || s->form != EDG_FORM_STORED) && (up ? tile_smem(dim, 0, 0, 0) > kTileSmemMax : !s->up.t16))
+    return EDG_OK;
   std::vector<uint32_t> off(dim + 1);
   EDG_CUDA(cudaMemcpyAsync(off.data(), B.off.p, (dim + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   EDG_CUDA(cudaStreamSynchronize(st));
@@ -1159,11 +1167,17 @@ int build_sell(edg_sector_s* s, SpinBasis& B, bool up) {
     EDG_CUDA(cudaStreamSynchronize(st));
   }
   std::vector<uint32_t> soff(nsl + 1, 0);
+  uint64_t padded = 0;
   for (int64_t sl = 0; sl < nsl; ++sl) {
     uint32_t w = 0;
     for (int64_t r = sl * 32; r < std::min<int64_t>(dim, sl * 32 + 32); ++r) w = std::max(w, off[r + 1] - off[r]);
     w = (w + kSellBatch - 1) / kSellBatch * kSellBatch;
-    soff[sl + 1] = soff[sl] + 32 * w;
+    padded += 32 * w;
+    soff[sl + 1] = uint32_t(padded);
+  }
+  if (!table_fits(padded)) {
+    set_error("SELL copy of a hop table: %llu entries, offsets are 32-bit", (unsigned long long)padded);
+    return EDG_ERR_UNSUPPORTED;
   }
   // entry: bit 31 = sign (uniform tables), bits 0..30 = source; padding points at the
   // zero slot dim that the up pass keeps after the staged rows
@@ -1282,6 +1296,58 @@ int sector_variant_tables(edg_sector_s* s) {
   return EDG_OK;
 }
 
+namespace {
+
+// Whether the H x v of this direct-form sector reads its tables, in either precision (hxv_apply).
+bool direct_reads_tables(const edg_sector_s* s) {
+  const int W = s->cplx ? 2 : 1;
+  for (size_t real : {sizeof(float), sizeof(double)}) {
+    const int64_t most = s->cplx ? kFusedMaxDimC : real == 8 ? kFusedMaxDim64 : kFusedMaxDim32;
+    if (s->dim <= most && tile_available(s, W * real, true)) return true;
+    if (s->dw.max_row <= kDwHops && s->dw.groups > 0 && tile_available(s, W * real, false)) return true;
+  }
+  return false;
+}
+
+void drop_tables(SpinBasis& B) {
+  B.off.reset();
+  B.src.reset();
+  B.val64.reset();
+  B.val32.reset();
+  B.val64i.reset();
+  B.val32i.reset();
+  B.group_off.reset();
+  B.group_rows.reset();
+  for (int o = 0; o < 2; ++o) {
+    B.t16_ent[o].reset();
+    B.t16_off[o].reset();
+  }
+  B.t16_code.reset();
+  B.t16_pal.reset();
+  B.nnz = 0;
+  B.max_row = B.groups = B.group_max = 0;
+  B.t16 = false;
+}
+
+// The tables of a direct-form sector, where the row tiles will read them; without them, for want
+// of memory too, the bitstring kernels apply H.
+int build_direct_tables(edg_sector_s* s) {
+  const int ns = s->model.ns;
+  if (!direct_tables(s->up.dim, s->dw.dim, hop_total(ns, s->nup, s->bonds[0].nb),
+                     hop_total(ns, s->ndw, s->bonds[1].nb), s->cplx))
+    return EDG_OK;
+  int st = build_tables(s, 1, s->up);
+  if (st == EDG_OK && s->up.t16) st = build_tables(s, 2, s->dw);
+  if (st != EDG_OK && st != EDG_ERR_NOMEM) return st;
+  if (st != EDG_OK || !direct_reads_tables(s)) {
+    drop_tables(s->up);
+    drop_tables(s->dw);
+  }
+  return EDG_OK;
+}
+
+}  // namespace
+
 int sector_build(edg_sector_s* s) {
   // exact binomial table C(n,k), n,k < kBinomN
   std::vector<uint32_t> C(kBinomN * kBinomN, 0);
@@ -1294,10 +1360,12 @@ int sector_build(edg_sector_s* s) {
   s->dim = s->up.dim * s->dw.dim;
   s->vlen = s->cplx ? 2 * s->dim : s->dim;
   s->U = s->model.uloc;
-  EDG_CHECK(build_tables(s, 1, s->up));
-  EDG_CHECK(build_tables(s, 2, s->dw));
-  if (s->form != EDG_FORM_STORED) {
-    // direct form: also the bond lists (both spins packed: [spin][k] -> a,b ; values)
+  if (s->form == EDG_FORM_STORED) {
+    EDG_CHECK(build_tables(s, 1, s->up));
+    EDG_CHECK(build_tables(s, 2, s->dw));
+  } else {
+    EDG_CHECK(build_direct_tables(s));
+    // the bond lists (both spins packed: [spin][k] -> a,b ; values)
     std::vector<int32_t> hb;
     std::vector<double> hv, hvi;
     for (int sp = 0; sp < 2; ++sp) {

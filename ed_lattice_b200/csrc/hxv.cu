@@ -769,8 +769,6 @@ __global__ void __launch_bounds__(256) k_hxv_fused(HxvArgs<T> a, int64_t ntiles)
 // each slab. Equal work per CTA keeps the whole grid within a few slabs of each other, so
 // the slab being combined (DimDw rows x 32*VEC columns) stays in L2 while each of its rows
 // is read once per hop; no global load of the hop list sits in the inner loop.
-constexpr int kDwHops = 32;  // hop-list capacity per row held in shared memory
-
 template <typename T, int VEC, int NSEG, int KU, int PARTS, bool FIRST, bool SCALED, int W = 1>
 __global__ void __launch_bounds__(256, 4) k_dw_grp(HxvArgs<T> a, const uint32_t* __restrict__ goff,
                                                 const uint32_t* __restrict__ grows, int64_t nslab,

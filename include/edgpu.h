@@ -42,8 +42,11 @@ enum {
  * src/DIAG/HAMILTONIAN.f90:148-160). STORED = spMatVec over tables built once per sector;
  * DIRECT = directMatVec: its summation order (diagonal, up, down), its use of Hij without
  * conjugation and its ed_filling rule for the diagonal. The tables of one spin take O(DimUp) or
- * O(DimDw) bytes, so both forms run from them; matrix elements are generated on the fly only
- * for rows beyond shared memory or more than 32 hops per row. */
+ * O(DimDw) bytes, so both forms run from them. DIRECT builds them only where they are read and
+ * take little beside a vector; rows beyond shared memory (DimUp above 14,343), more than 32 hops
+ * per row in a large sector and very many configurations of one spin beside few of the other
+ * are applied from the bitstrings, without tables. STORED refuses (EDG_ERR_UNSUPPORTED) a spin
+ * of 2^32 hops or more. */
 enum { EDG_FORM_STORED = 0, EDG_FORM_DIRECT = 1 };
 
 /* Precision of the device Lanczos vectors. Scalars (alpha, beta, dots) are always FP64. */

@@ -1,11 +1,27 @@
 """Columns H e_i of a sector by the definition, for sectors too large for the oracle's H x v: the
 hops of one bitstring pair, with hopping values that products and sums keep exact."""
+import math
+
 import numpy as np
 
-from oracle import oracle as O
+
+def _rank(m):
+    """Place of the bitstring m among those with as many bits, ascending."""
+    bits = [b for b in range(m.bit_length()) if (m >> b) & 1]
+    return sum(math.comb(b, k + 1) for k, b in enumerate(bits))
 
 
-def _hops(h, m, states, conj):
+def _state(r, ns, n):
+    """The bitstring of rank r among those of n bits in ns."""
+    m = 0
+    for k in range(n, 0, -1):
+        b = max(c for c in range(ns) if math.comb(c, k) <= r)
+        m |= 1 << b
+        r -= math.comb(b, k)
+    return m
+
+
+def _hops(h, m, conj):
     """(rank of the target, value) of sum_ab h[a, b] c+_a c_b on the bitstring m."""
     ns = h.shape[0]
     out = []
@@ -17,7 +33,7 @@ def _hops(h, m, states, conj):
             between = (m >> (lo + 1)) & ((1 << (hi - lo - 1)) - 1)
             t = m - (1 << b) + (1 << a)
             v = h[a, b].conjugate() if conj else h[a, b]
-            out.append((int(np.searchsorted(states, t)), -v if bin(between).count("1") & 1 else v))
+            out.append((_rank(t), -v if bin(between).count("1") & 1 else v))
     return out
 
 
@@ -27,19 +43,19 @@ class Columns:
 
     def __init__(self, h, nup, ndw, uloc, xmu, stored=True):
         self.h, self.u, self.xmu, self.stored = h, uloc, xmu, stored
-        self.up, self.dw = O.build_map(h.shape[0], nup), O.build_map(h.shape[0], ndw)
-        self.ne = nup + ndw
+        self.ns, self.nup, self.ndw = h.shape[0], nup, ndw
+        self.dimup = math.comb(self.ns, nup)
 
     def __call__(self, i):
-        iup, idw = i % self.up.size, i // self.up.size
-        mu, md = int(self.up[iup]), int(self.dw[idw])
+        iup, idw = i % self.dimup, i // self.dimup
+        mu, md = _state(iup, self.ns, self.nup), _state(idw, self.ns, self.ndw)
         conj = self.stored and np.iscomplexobj(self.h)
-        col = {i: self.u * bin(mu & md).count("1") - self.xmu * self.ne}
-        for t, v in _hops(self.h, mu, self.up, conj):
-            j = t + idw * self.up.size
+        col = {i: self.u * bin(mu & md).count("1") - self.xmu * (self.nup + self.ndw)}
+        for t, v in _hops(self.h, mu, conj):
+            j = t + idw * self.dimup
             col[j] = col.get(j, 0) + v
-        for t, v in _hops(self.h, md, self.dw, conj):
-            j = iup + t * self.up.size
+        for t, v in _hops(self.h, md, conj):
+            j = iup + t * self.dimup
             col[j] = col.get(j, 0) + v
         return {j: v for j, v in col.items() if v != 0}
 

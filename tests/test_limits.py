@@ -19,6 +19,11 @@ SHIM = r"""
 using namespace edg;
 extern "C" {
 int down_index(int64_t dim) { return tile_down_index(dim); }
+uint64_t hops(int ns, int nel, int64_t bonds) { return hop_total(ns, nel, bonds); }
+int fits(uint64_t n) { return table_fits(n); }
+int direct(int64_t dimup, int64_t dimdw, uint64_t hu, uint64_t hd, int cplx) {
+  return direct_tables(dimup, dimdw, hu, hd, cplx != 0);
+}
 }
 """
 
@@ -32,6 +37,9 @@ def rules(tmp_path_factory):
                     "-I" + os.path.join(ROOT, "ed_lattice_b200", "csrc"), str(src), "-o", str(lib)], check=True)
     r = C.CDLL(str(lib))
     r.down_index.argtypes = [C.c_int64]
+    r.hops.argtypes, r.hops.restype = [C.c_int, C.c_int, C.c_int64], C.c_uint64
+    r.fits.argtypes = [C.c_uint64]
+    r.direct.argtypes = [C.c_int64, C.c_int64, C.c_uint64, C.c_uint64, C.c_int]
     return r
 
 
@@ -60,3 +68,32 @@ def test_tile_down_hops_fit_their_index(rules):
         dim = math.comb(ns, nup) * math.comb(ns, ndw)
         last = (math.comb(ns, ndw) - 1) * math.comb(ns, nup)  # the last row's first element
         assert bool(rules.down_index(dim)) == fits == (last < 2**31)
+
+
+def _bonds(h):
+    return np.count_nonzero(h) - np.count_nonzero(np.diag(h))
+
+
+def test_hop_totals(rules):
+    """The 64-bit count against the tables that the oracle builds, and past 2^32 by the binomials."""
+    for lx, ly in ((1, 1), (2, 1), (8, 1), (3, 3)):
+        h = E.square_lattice(lx, ly) if lx * ly > 1 else np.zeros((1, 1))
+        ns = lx * ly
+        for nel in range(ns + 1):
+            assert rules.hops(ns, nel, _bonds(h)) == O.hop_csr(O.Model(h), 1, nel)[1].size
+    n = rules.hops(30, 15, _bonds(E.square_lattice(5, 6)))
+    assert n == 120 * math.comb(28, 14) and not rules.fits(n)
+    assert rules.fits(2**32 - 2) and not rules.fits(2**32 - 1) and not rules.fits(2**32)
+
+
+@pytest.mark.parametrize("case", [(5, 6, 15, 0, 0, False), (5, 6, 0, 15, 1, False),  # 4.8e9 hops of a spin
+                                  (30, 1, 15, 1, 0, False), (30, 1, 1, 15, 0, False),  # 37 GB of tables
+                                  (22, 1, 1, 11, 0, False), (22, 1, 1, 11, 1, False),  # more than the vector
+                                  (9, 2, 9, 2, 0, False), (9, 2, 9, 2, 1, False),  # rows beyond the tiles
+                                  (4, 4, 6, 6, 0, True), (4, 4, 8, 8, 1, True), (8, 1, 4, 4, 0, True),
+                                  (9, 2, 2, 9, 1, True), (9, 2, 0, 9, 0, True), (3, 4, 6, 6, 0, True)])
+def test_direct_form_tables(rules, case):
+    lx, ly, nup, ndw, cplx, want = case
+    ns, nb = lx * ly, _bonds(E.square_lattice(lx, ly))
+    assert bool(rules.direct(math.comb(ns, nup), math.comb(ns, ndw), rules.hops(ns, nup, nb),
+                             rules.hops(ns, ndw, nb), cplx)) == want
