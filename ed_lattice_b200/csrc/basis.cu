@@ -1096,6 +1096,50 @@ int build_variants(edg_sector_s* s, SpinBasis& B) {
   return EDG_OK;
 }
 
+// LPT grouping of rows (`order`: most hops first) for the down-spin pass in one precision; FP32 gets
+// none of its own where it would have as many groups as FP64.
+int build_groups(edg_sector_s* s, const SpinBasis& B, const std::vector<uint32_t>& off,
+                 const std::vector<uint32_t>& order, size_t real, SpinBasis::RowGroups& g) {
+  cudaStream_t st = s->stream;
+  const int64_t dim = B.dim;
+  const int W = s->cplx ? 2 : 1;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t G = dw_group_count(dim, int64_t(sms) * 4, real, W);
+  if (real == sizeof(float) && G == B.grp[0].count) return EDG_OK;
+  const size_t most = size_t(dw_group_most(real, W));
+  std::vector<std::pair<int64_t, int64_t>> heap;  // (load, group) min-heap
+  for (int64_t i = 0; i < G; ++i) heap.push_back({0, i});
+  auto cmp = [](const std::pair<int64_t, int64_t>& x, const std::pair<int64_t, int64_t>& y) { return x > y; };
+  std::make_heap(heap.begin(), heap.end(), cmp);
+  std::vector<std::vector<uint32_t>> members(G);
+  for (uint32_t r : order) {
+    std::pop_heap(heap.begin(), heap.end(), cmp);
+    auto& top = heap.back();
+    members[top.second].push_back(r);
+    top.first += 1 + int64_t(off[r + 1] - off[r]);  // diagonal + hops
+    if (members[top.second].size() < most) std::push_heap(heap.begin(), heap.end(), cmp);
+    else heap.pop_back();  // full
+  }
+  std::vector<uint32_t> goff(G + 1, 0), grows;
+  grows.reserve(dim);
+  g.max = 0;
+  for (int64_t i = 0; i < G; ++i) {
+    std::sort(members[i].begin(), members[i].end());
+    grows.insert(grows.end(), members[i].begin(), members[i].end());
+    goff[i + 1] = uint32_t(grows.size());
+    g.max = std::max<int>(g.max, int(members[i].size()));
+  }
+  g.count = int(G);
+  EDG_CHECK(g.off.alloc(G + 1, st, "row groups"));
+  EDG_CHECK(g.rows.alloc(grows.size() + 1, st, "row groups"));
+  EDG_CUDA(cudaMemcpyAsync(g.off.p, goff.data(), goff.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+  EDG_CUDA(cudaMemcpyAsync(g.rows.p, grows.data(), grows.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+  EDG_CUDA(cudaStreamSynchronize(st));
+  return EDG_OK;
+}
+
 // Work split of the down pass and, for the up spin, the schedules of the up pass: the tile
 // kernels' 16-bit slots or, for rows and tables those do not take, the SELL-32 copy. Built on the
 // host from the device CSR (the tables are O(DimUp), about 1 MB for a 4x4 lattice, so this is a
@@ -1112,43 +1156,14 @@ int build_sell(edg_sector_s* s, SpinBasis& B, bool up) {
   const int64_t nsl = (dim + 31) / 32;
   B.max_row = 0;
   for (int64_t r = 0; r < dim; ++r) B.max_row = std::max<int>(B.max_row, int(off[r + 1] - off[r]));
-  // LPT grouping of rows for the down-spin pass: one group per resident CTA (4 per SM)
   if (!up) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t G = std::max<int64_t>(1, std::min<int64_t>(int64_t(sms) * 4, dim));
-    std::vector<int64_t> order(dim);
-    for (int64_t r = 0; r < dim; ++r) order[r] = r;
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int64_t x, int64_t y) { return off[x + 1] - off[x] > off[y + 1] - off[y]; });
-    std::vector<std::pair<int64_t, int64_t>> heap;  // (load, group) min-heap
-    for (int64_t g = 0; g < G; ++g) heap.push_back({0, g});
-    auto cmp = [](const std::pair<int64_t, int64_t>& x, const std::pair<int64_t, int64_t>& y) { return x > y; };
-    std::make_heap(heap.begin(), heap.end(), cmp);
-    std::vector<std::vector<uint32_t>> members(G);
-    for (int64_t r : order) {
-      std::pop_heap(heap.begin(), heap.end(), cmp);
-      auto& top = heap.back();
-      members[top.second].push_back(uint32_t(r));
-      top.first += 1 + int64_t(off[r + 1] - off[r]);  // diagonal + hops
-      std::push_heap(heap.begin(), heap.end(), cmp);
-    }
-    std::vector<uint32_t> goff(G + 1, 0), grows;
-    grows.reserve(dim);
-    B.group_max = 0;
-    for (int64_t g = 0; g < G; ++g) {
-      std::sort(members[g].begin(), members[g].end());
-      grows.insert(grows.end(), members[g].begin(), members[g].end());
-      goff[g + 1] = uint32_t(grows.size());
-      B.group_max = std::max<int>(B.group_max, int(members[g].size()));
-    }
-    B.groups = int(G);
-    EDG_CHECK(B.group_off.alloc(G + 1, st, "row groups"));
-    EDG_CHECK(B.group_rows.alloc(grows.size() + 1, st, "row groups"));
-    EDG_CUDA(cudaMemcpyAsync(B.group_off.p, goff.data(), goff.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-    EDG_CUDA(cudaMemcpyAsync(B.group_rows.p, grows.data(), grows.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-    EDG_CUDA(cudaStreamSynchronize(st));
+    std::vector<int64_t> at(B.max_row + 2, 0);  // rows of more hops than h, at[B.max_row - h]
+    for (int64_t r = 0; r < dim; ++r) ++at[B.max_row - int(off[r + 1] - off[r]) + 1];
+    for (int h = 1; h <= B.max_row; ++h) at[h] += at[h - 1];
+    std::vector<uint32_t> order(dim);
+    for (int64_t r = 0; r < dim; ++r) order[at[B.max_row - int(off[r + 1] - off[r])]++] = uint32_t(r);
+    EDG_CHECK(build_groups(s, B, off, order, sizeof(double), B.grp[0]));
+    EDG_CHECK(build_groups(s, B, off, order, sizeof(float), B.grp[1]));
   }
   const BondList& bl = s->bonds[up ? 0 : 1];
   const double hsgn = bl.nb ? bl.h[0] : 0.0;  // value encoded by code 0
@@ -1304,7 +1319,7 @@ bool direct_reads_tables(const edg_sector_s* s) {
   for (size_t real : {sizeof(float), sizeof(double)}) {
     const int64_t most = s->cplx ? kFusedMaxDimC : real == 8 ? kFusedMaxDim64 : kFusedMaxDim32;
     if (s->dim <= most && tile_available(s, W * real, true)) return true;
-    if (s->dw.max_row <= kDwHops && s->dw.groups > 0 && tile_available(s, W * real, false)) return true;
+    if (s->dw.max_row <= kDwHops && s->dw.grp[0].count > 0 && tile_available(s, W * real, false)) return true;
   }
   return false;
 }
@@ -1316,8 +1331,11 @@ void drop_tables(SpinBasis& B) {
   B.val32.reset();
   B.val64i.reset();
   B.val32i.reset();
-  B.group_off.reset();
-  B.group_rows.reset();
+  for (auto& g : B.grp) {
+    g.off.reset();
+    g.rows.reset();
+    g.count = g.max = 0;
+  }
   for (int o = 0; o < 2; ++o) {
     B.t16_ent[o].reset();
     B.t16_off[o].reset();
@@ -1325,7 +1343,7 @@ void drop_tables(SpinBasis& B) {
   B.t16_code.reset();
   B.t16_pal.reset();
   B.nnz = 0;
-  B.max_row = B.groups = B.group_max = 0;
+  B.max_row = 0;
   B.t16 = false;
 }
 

@@ -192,8 +192,6 @@ struct SpinBasis {
   DevBuf<double> split_v64;     // only when !sell_uniform
   DevBuf<float> split_v32;
   int max_row = 0;              // longest hop list of any configuration
-  // Down-spin pass work split: rows grouped into `groups` CTAs with near-equal total hop
-  // counts (longest-processing-time-first assignment), CSR: group_off[groups+1], group_rows.
   // Contiguous row blocks for the block-staged down pass, one CTA each: block g owns rows
   // [off[g], off[g+1]), blocks balanced by hop count; rowblk[0] for 1024-thread CTAs (about
   // one per SM), rowblk[1] for 512-thread CTAs (about two per SM).
@@ -203,10 +201,17 @@ struct SpinBasis {
     int max_rows = 0;
   };
   RowBlocks rowblk[2];
-  DevBuf<uint32_t> group_off;
-  DevBuf<uint32_t> group_rows;
-  int groups = 0;
-  int group_max = 0;            // most rows in one group
+  // Down-spin pass work split: rows grouped into `count` CTAs with near-equal total hop counts
+  // (longest-processing-time-first assignment), CSR: off[count+1], rows; `max` rows in the largest.
+  // FP32 has its own where its smaller rows want fewer groups (dw_group_count).
+  struct RowGroups {
+    DevBuf<uint32_t> off;
+    DevBuf<uint32_t> rows;
+    int count = 0;
+    int max = 0;
+  };
+  RowGroups grp[2];
+  const RowGroups& groups(size_t real) const { return grp[real == 4 && grp[1].count ? 1 : 0]; }
   // Kronecker schedule of the FP32 up pass (uniform real tables). The sites split at bit
   // kron_m into a low part (bits below kron_m) and a high part. Ascending order keeps the
   // configurations of one high part h together: a block of consecutive columns, one per low

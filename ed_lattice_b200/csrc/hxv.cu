@@ -1376,11 +1376,11 @@ int launch_dw_grp(const HxvArgs<T>& a, const SpinBasis& Bdw, bool v2, cudaStream
   constexpr int NSEG = F32 ? 4 : 2;
   auto kern = v2 ? k_dw_grp<T, 2, NSEG, F32 && !SCALED ? 2 : 3, F32 ? 1 : 2, FIRST, SCALED>
                  : k_dw_grp<T, 1, 4, F32 ? 4 : 3, F32 ? 2 : 1, FIRST, SCALED>;
-  const size_t smem = size_t(Bdw.group_max) * (kDwHops * (sizeof(T) + 4) + sizeof(T) + 12) + 16;
+  const SpinBasis::RowGroups& g = Bdw.groups(sizeof(T));
+  const size_t smem = dw_group_smem(g.max, sizeof(T), 1);
   if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   const int64_t slab = v2 ? 64 * NSEG * (F32 ? 1 : 2) : 128 * (F32 ? 2 : 1);
-  kern<<<dim3(Bdw.groups, a.ncols), 256, smem, st>>>(a, Bdw.group_off.p, Bdw.group_rows.p, (a.dimup + slab - 1) / slab,
-                                                      nullptr);
+  kern<<<dim3(g.count, a.ncols), 256, smem, st>>>(a, g.off.p, g.rows.p, (a.dimup + slab - 1) / slab, nullptr);
   EDG_CUDA(cudaGetLastError());
   return EDG_OK;
 }
@@ -1419,7 +1419,7 @@ int dw_pass(const HxvArgs<T>& a, const SpinBasis& Bdw, cudaStream_t st, int sms)
       return EDG_OK;
     }
   }
-  if (Bdw.max_row <= kDwHops && Bdw.groups > 0) return launch_dw_grp<T, FIRST, SCALED>(a, Bdw, v2, st);
+  if (Bdw.max_row <= kDwHops && Bdw.grp[0].count > 0) return launch_dw_grp<T, FIRST, SCALED>(a, Bdw, v2, st);
   if (SCALED || a.ncols > 1) {
     set_error("fused Lanczos and block H x V need the grouped down pass");
     return EDG_ERR_UNSUPPORTED;
@@ -1441,10 +1441,11 @@ template <typename T, bool FIRST>
 int dw_pass_c(const HxvArgs<T>& a, const SpinBasis& Bdw, const T* vi_dw, cudaStream_t st) {
   constexpr int NSEG = sizeof(T) == 4 ? 4 : 2, PARTS = 2;
   auto kern = k_dw_grp<T, 2, NSEG, 2, PARTS, FIRST, false, 2>;
-  const size_t smem = size_t(Bdw.group_max) * (kDwHops * (2 * sizeof(T) + 4) + sizeof(T) + 12) + 16;
+  const SpinBasis::RowGroups& g = Bdw.groups(sizeof(T));
+  const size_t smem = dw_group_smem(g.max, sizeof(T), 2);
   if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   const int64_t slab = 32 * NSEG * PARTS, nslab = (a.dimup + slab - 1) / slab;
-  kern<<<dim3(Bdw.groups, 1), 256, smem, st>>>(a, Bdw.group_off.p, Bdw.group_rows.p, nslab, vi_dw);
+  kern<<<dim3(g.count, 1), 256, smem, st>>>(a, g.off.p, g.rows.p, nslab, vi_dw);
   EDG_CUDA(cudaGetLastError());
   return EDG_OK;
 }
@@ -1640,7 +1641,7 @@ int hxv_apply(edg_sector_s* s, const T* v, T* hv) {
     const bool vec = reinterpret_cast<uintptr_t>(v) % (2 * sizeof(T)) == 0 && reinterpret_cast<uintptr_t>(hv) % (2 * sizeof(T)) == 0;
     if (vec && s->dim <= kFusedMaxDimC && tile_available(s, 2 * sizeof(T), true))
       return tile_cplx<T>(a, s->up, s->dw, vi, stored ? TileForm::kDwUp : TileForm::kUpDw, st, sms);
-    if (vec && s->dw.max_row <= kDwHops && s->dw.groups > 0 && tile_available(s, 2 * sizeof(T), false)) {
+    if (vec && s->dw.max_row <= kDwHops && s->dw.grp[0].count > 0 && tile_available(s, 2 * sizeof(T), false)) {
       if (stored) {
         EDG_CHECK((dw_pass_c<T, true>(a, s->dw, vi, st)));
         return tile_cplx<T>(a, s->up, s->dw, nullptr, TileForm::kUpAdd, st, sms);
@@ -1675,7 +1676,7 @@ int hxv_apply(edg_sector_s* s, const T* v, T* hv) {
     // whose up gathers scatter over global memory; 3x4 (6,6) 25 / 19 us against 126 / 119). The bitstring kernels serve the rows and hop lists that those do not take.
     if (s->dim <= (sizeof(T) == 8 ? kFusedMaxDim64 : kFusedMaxDim32) && tile_available(s, sizeof(T), true))
       return tile_real<T>(a, s->up, s->dw, TileForm::kUpDw, false, st, sms);
-    if (s->dw.max_row <= kDwHops && s->dw.groups > 0 && tile_available(s, sizeof(T), false)) {
+    if (s->dw.max_row <= kDwHops && s->dw.grp[0].count > 0 && tile_available(s, sizeof(T), false)) {
       EDG_CHECK((tile_real<T>(a, s->up, s->dw, TileForm::kUp, false, st, sms)));
       return dw_add<T>(a, s->dw, st);
     }
@@ -1753,7 +1754,7 @@ template <typename T>
 int hxv_apply_lz(edg_sector_s* s, const T* u, const T* uprev, T* w, const double* bn, int j, double* partial,
                  double* aout) {
   if (s->cplx || s->form != EDG_FORM_STORED || up_rows_per_cta(s->up.dim, sizeof(T)) == 0 ||
-      s->dw.max_row > kDwHops || s->dw.groups == 0) {
+      s->dw.max_row > kDwHops || s->dw.grp[0].count == 0) {
     set_error("fused Lanczos H x v not available for this sector");
     return EDG_ERR_UNSUPPORTED;
   }
@@ -1771,7 +1772,7 @@ int hxv_apply_lz(edg_sector_s* s, const T* u, const T* uprev, T* w, const double
 }
 bool hxv_lz_available(const edg_sector_s* s, size_t elem) {
   return !s->cplx && s->form == EDG_FORM_STORED && up_rows_per_cta(s->up.dim, elem) > 0 &&
-         s->dw.max_row <= kDwHops && s->dw.groups > 0;
+         s->dw.max_row <= kDwHops && s->dw.grp[0].count > 0;
 }
 template <typename T>
 int hxv_block(edg_sector_s* s, int ncols, const int* active, const T* v, T* hv) {

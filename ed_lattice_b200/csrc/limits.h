@@ -47,4 +47,25 @@ inline bool direct_tables(int64_t dimup, int64_t dimdw, uint64_t hops_up, uint64
   return (hops_up + hops_dw) * (cplx ? 28 : 16) <= room;
 }
 
+
+// ---- row groups of the grouped down pass (k_dw_grp)
+// Shared memory of a row of a group: its hop values (W reals each) and sources, its diagonal term,
+// index, configuration and hop count.
+inline size_t dw_row_smem(size_t real, int W) { return size_t(kDwHops) * (W * real + 4) + real + 12; }
+inline size_t dw_group_smem(int64_t rows, size_t real, int W) { return size_t(rows) * dw_row_smem(real, W) + 16; }
+// Most rows of a group: four blocks per SM stay resident.
+constexpr size_t kDwGroupSmem = 52 * 1024;
+inline int64_t dw_group_most(size_t real, int W) { return int64_t((kDwGroupSmem - 16) / dw_row_smem(real, W)); }
+// Number of groups: one per resident block, all of them at work on the same slab of columns, or,
+// where those would be larger (from 73,000 FP64 rows, 44,000 complex128), as many for each of
+// several turns, with a sixteenth of room to even out their hops. ms per H x v with one group per
+// resident block whatever its size (one block per SM of 200 KB at the most, a failed launch
+// beyond) and now: 20-site ring (2,10), 184,756 rows, complex128 2.51 and 1.32, real FP64 1.42
+// and 0.65; 5x4 lattice (3,8), 125,970 rows, complex128 13.9 and 7.3, FP32 2.01 and 1.43.
+inline int64_t dw_group_count(int64_t dim, int64_t resident, size_t real, int W) {
+  const int64_t rows = dw_group_most(real, W) * 15 / 16;
+  if (dim <= resident) return dim < 1 ? 1 : dim;
+  return resident * ((dim + resident * rows - 1) / (resident * rows));
+}
+
 }  // namespace edg

@@ -19,6 +19,9 @@ SHIM = r"""
 using namespace edg;
 extern "C" {
 int down_index(int64_t dim) { return tile_down_index(dim); }
+int64_t groups(int64_t dim, int64_t resident, int real, int W) { return dw_group_count(dim, resident, real, W); }
+int64_t group_most(int real, int W) { return dw_group_most(real, W); }
+int64_t group_smem(int64_t rows, int real, int W) { return dw_group_smem(rows, real, W); }
 uint64_t hops(int ns, int nel, int64_t bonds) { return hop_total(ns, nel, bonds); }
 int fits(uint64_t n) { return table_fits(n); }
 int direct(int64_t dimup, int64_t dimdw, uint64_t hu, uint64_t hd, int cplx) {
@@ -38,6 +41,9 @@ def rules(tmp_path_factory):
     r = C.CDLL(str(lib))
     r.down_index.argtypes = [C.c_int64]
     r.hops.argtypes, r.hops.restype = [C.c_int, C.c_int, C.c_int64], C.c_uint64
+    r.groups.argtypes, r.groups.restype = [C.c_int64, C.c_int64, C.c_int, C.c_int], C.c_int64
+    r.group_most.argtypes, r.group_most.restype = [C.c_int, C.c_int], C.c_int64
+    r.group_smem.argtypes, r.group_smem.restype = [C.c_int64, C.c_int, C.c_int], C.c_int64
     r.fits.argtypes = [C.c_uint64]
     r.direct.argtypes = [C.c_int64, C.c_int64, C.c_uint64, C.c_uint64, C.c_int]
     return r
@@ -97,3 +103,18 @@ def test_direct_form_tables(rules, case):
     ns, nb = lx * ly, _bonds(E.square_lattice(lx, ly))
     assert bool(rules.direct(math.comb(ns, nup), math.comb(ns, ndw), rules.hops(ns, nup, nb),
                              rules.hops(ns, ndw, nb), cplx)) == want
+
+
+@pytest.mark.parametrize("W", [1, 2])
+@pytest.mark.parametrize("real", [4, 8])
+def test_row_groups_fit_shared_memory(rules, real, W):
+    """Every number of down configurations has room in its groups, and four blocks with a group each
+    and 4 KB of static arrays in an SM's 228 KB (1 KB of it reserved per block)."""
+    most = rules.group_most(real, W)
+    assert 4 * (rules.group_smem(most, real, W) + 4096 + 1024) <= 228 * 1024
+    dims = {math.comb(n, k) for n in range(1, 31) for k in range(n + 1)}
+    dims |= {592 * k * most + d for k in (1, 2, 15) for d in (-1, 0, 1)} | {206_600, 335_700}
+    for dim in dims:
+        g = rules.groups(dim, 592, real, W)
+        assert 1 <= g <= dim and (g % 592 == 0 or g == dim < 592)
+        assert g * most >= dim
