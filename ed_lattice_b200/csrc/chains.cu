@@ -170,8 +170,7 @@ int poles_weights_block(cudaStream_t st, int k, int nlanc, const double* alanc, 
   // one warp per chain; its three arrays in shared memory up to nlanc = 9,400
   const size_t smem = size_t(3) * nlanc * sizeof(double);
   const bool in_smem = smem <= size_t(227) * 1024;
-  if (in_smem && smem > 48 * 1024)
-    EDG_CUDA(cudaFuncSetAttribute(k_poles_ql, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  if (in_smem) EDG_CHECK(allow_smem(k_poles_ql, smem));
   k_poles_ql<<<k, 32, in_smem ? smem : 0, st>>>(k, nlanc, da, db, dns, dn2, ei, isign, in_smem, dwork, dp, dw,
                                                 dstat);
   EDG_CUDA(cudaGetLastError());

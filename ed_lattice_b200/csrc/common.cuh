@@ -36,6 +36,20 @@ const char* get_error();
     if (s_ != EDG_OK) return s_; \
   } while (0)
 
+// Lets `kern` be launched with `smem` bytes of dynamic shared memory. The limit belongs to the
+// function, which all host threads share: every call sets the same one, the most that the kernel's
+// static arrays leave, so that no thread lowers it between another one's call and launch. (The
+// default, 48 KB with the static arrays, holds for less than 32.)
+template <typename... A>
+int allow_smem(void (*kern)(A...), size_t smem) {
+  if (smem <= 32 * 1024) return EDG_OK;
+  cudaFuncAttributes at{};
+  EDG_CUDA(cudaFuncGetAttributes(&at, kern));
+  EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                int(kSmemPerBlock - at.sharedSizeBytes)));
+  return EDG_OK;
+}
+
 // Makes a sector's device current for the rest of the enclosing scope and gives the caller
 // back its own current device on every return path: a host code that drives several GPUs
 // from one thread must find its current device unchanged after any library call.

@@ -1350,7 +1350,7 @@ int launch_up_smem(const HxvArgs<T>& a, const SellArgs<T>& sl, cudaStream_t st, 
   const size_t smem = size_t(a.dimup + kUpZeroSlots) * RT * sizeof(T);
   const int per_sm = smem <= kUpSmemTwoPerSM ? 2 : 1;
   auto kern = per_sm == 2 ? k_up_smem<T, RT, FIRST, UNIFORM, LZ, false> : k_up_smem<T, RT, FIRST, UNIFORM, LZ, true>;
-  if (smem > 48 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  EDG_CHECK(allow_smem(kern, smem));
   const int64_t nrb = (a.dimdw + RT - 1) / RT;
   int64_t g = nrb < int64_t(sms) * per_sm ? nrb : int64_t(sms) * per_sm;
   if (LZ && g > kRedBlocks) g = kRedBlocks;  // one partial per block in the reduction scratch
@@ -1378,7 +1378,7 @@ int launch_dw_grp(const HxvArgs<T>& a, const SpinBasis& Bdw, bool v2, cudaStream
                  : k_dw_grp<T, 1, 4, F32 ? 4 : 3, F32 ? 2 : 1, FIRST, SCALED>;
   const SpinBasis::RowGroups& g = Bdw.groups(sizeof(T));
   const size_t smem = dw_group_smem(g.max, sizeof(T), 1);
-  if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  EDG_CHECK(allow_smem(kern, smem));
   const int64_t slab = v2 ? 64 * NSEG * (F32 ? 1 : 2) : 128 * (F32 ? 2 : 1);
   kern<<<dim3(g.count, a.ncols), 256, smem, st>>>(a, g.off.p, g.rows.p, (a.dimup + slab - 1) / slab, nullptr);
   EDG_CUDA(cudaGetLastError());
@@ -1412,7 +1412,7 @@ int dw_pass(const HxvArgs<T>& a, const SpinBasis& Bdw, cudaStream_t st, int sms)
     if (smem <= (nt == 512 ? kUpSmemTwoPerSM : kUpSmemOnePerSM)) {
       auto kern = nt == 512 ? (v2 ? k_dw_blk<T, 2, NSEG, KU, FIRST, SCALED, 512> : k_dw_blk<T, 1, NSEG, KU, FIRST, SCALED, 512>)
                             : (v2 ? k_dw_blk<T, 2, NSEG, KU, FIRST, SCALED, 1024> : k_dw_blk<T, 1, NSEG, KU, FIRST, SCALED, 1024>);
-      EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      EDG_CHECK(allow_smem(kern, smem));
       const int64_t nslab = (a.dimup + slabw - 1) / slabw;
       kern<<<dim3(rb->count, a.ncols), nt, smem, st>>>(a, rb->off.p, nslab);
       EDG_CUDA(cudaGetLastError());
@@ -1443,7 +1443,7 @@ int dw_pass_c(const HxvArgs<T>& a, const SpinBasis& Bdw, const T* vi_dw, cudaStr
   auto kern = k_dw_grp<T, 2, NSEG, 2, PARTS, FIRST, false, 2>;
   const SpinBasis::RowGroups& g = Bdw.groups(sizeof(T));
   const size_t smem = dw_group_smem(g.max, sizeof(T), 2);
-  if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  EDG_CHECK(allow_smem(kern, smem));
   const int64_t slab = 32 * NSEG * PARTS, nslab = (a.dimup + slab - 1) / slab;
   kern<<<dim3(g.count, 1), 256, smem, st>>>(a, g.off.p, g.rows.p, nslab, vi_dw);
   EDG_CUDA(cudaGetLastError());
@@ -1466,18 +1466,13 @@ bool launch_up_p16(const HxvArgs<float>& a, const SpinBasis& B, cudaStream_t st,
   const int per_sm = smem <= kUpSmemTwoPerSM ? 2 : 1;
   auto kern = neg ? (per_sm == 2 ? k_up_p16<true, false, LZ> : k_up_p16<true, true, LZ>)
                   : (per_sm == 2 ? k_up_p16<false, false, LZ> : k_up_p16<false, true, LZ>);
-  *status = EDG_OK;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  if (e != cudaSuccess) {
-    set_error("k_up_p16: %s", cudaGetErrorString(e));
-    *status = EDG_ERR_CUDA;
-    return true;
-  }
+  *status = allow_smem(kern, smem);
+  if (*status != EDG_OK) return true;
   const int64_t nrb = (a.dimdw + 1) / 2;
   int64_t g = nrb < int64_t(sms) * per_sm ? nrb : int64_t(sms) * per_sm;
   if (LZ && g > kRedBlocks) g = kRedBlocks;
   kern<<<dim3(int(g), a.ncols), 1024, smem, st>>>(a, q, nrb);
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("k_up_p16: %s", cudaGetErrorString(e));
     *status = EDG_ERR_CUDA;
@@ -1491,7 +1486,7 @@ int launch_up_kron_rt(const HxvArgs<float>& a, const KronArgs& q, cudaStream_t s
   const size_t smem = kron_smem(a.dimup, RT, q.nkrow, q.nhent);
   const int per_sm = smem <= kUpSmemTwoPerSM ? 2 : 1;
   auto kern = per_sm == 2 ? k_up_kron<RT, LZ, false> : k_up_kron<RT, LZ, true>;
-  if (smem > 48 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  EDG_CHECK(allow_smem(kern, smem));
   const int64_t nrb = (a.dimdw + RT - 1) / RT;
   int64_t g = nrb < int64_t(sms) * per_sm ? nrb : int64_t(sms) * per_sm;
   if (LZ && g > kRedBlocks) g = kRedBlocks;
@@ -1551,7 +1546,7 @@ int up_pass(const HxvArgs<T>& a, edg_sector_s* s, cudaStream_t st, int sms, int*
       for (int p = 0; p < B.split_parts; ++p) wmax = std::max<int64_t>(wmax, sp.col[p + 1] - sp.col[p]);
       const size_t smem = size_t(wmax + kUpZeroSlots) * sizeof(T);
       auto kern = B.sell_uniform ? k_up_split<T, FIRST, true> : k_up_split<T, FIRST, false>;
-      EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      EDG_CHECK(allow_smem(kern, smem));
       const int g = int(a.dimdw < int64_t(sms) ? a.dimdw : int64_t(sms));
       kern<<<g, 1024, smem, st>>>(a, sp);
       EDG_CUDA(cudaGetLastError());
@@ -1660,8 +1655,7 @@ int hxv_apply(edg_sector_s* s, const T* v, T* hv) {
       d.C = s->binom.p;
       const int nb = d.nb_up + d.nb_dw;
       const size_t smem = ((2 * nb * sizeof(int32_t) + 15) / 16) * 16 + 2 * nb * sizeof(T) + 16;
-      if (smem > 48 * 1024)
-        EDG_CUDA(cudaFuncSetAttribute(k_cplx_direct<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      EDG_CHECK(allow_smem(k_cplx_direct<T>, smem));
       k_cplx_direct<T><<<g, 256, smem, st>>>(a, d, s->bondhi_dev.p);
     }
     EDG_CUDA(cudaGetLastError());
@@ -1693,14 +1687,13 @@ int hxv_apply(edg_sector_s* s, const T* v, T* hv) {
     if (hop_bound <= kDirHops) {
       const int64_t nrb = (a.dimdw + kDirRows - 1) / kDirRows;
       const int g = int(nrb < int64_t(sms) * 8 ? nrb : int64_t(sms) * 8);
-      if (smem > 32 * 1024)
-        EDG_CUDA(cudaFuncSetAttribute(k_direct_rows<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      EDG_CHECK(allow_smem(k_direct_rows<T>, smem));
       k_direct_rows<T><<<g, 256, smem, st>>>(a, d, nrb);
     } else {
       const int64_t n = a.dimup * a.dimdw;
       const int64_t want = (n + 255) / 256;
       const int g = int(want < int64_t(sms) * 8 ? want : int64_t(sms) * 8);
-      if (smem > 48 * 1024) EDG_CUDA(cudaFuncSetAttribute(k_direct<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      EDG_CHECK(allow_smem(k_direct<T>, smem));
       k_direct<T><<<g, 256, smem, st>>>(a, d);
     }
     EDG_CUDA(cudaGetLastError());

@@ -7,6 +7,8 @@
 
 namespace edg {
 
+constexpr size_t kSmemPerBlock = 227 * 1024;  // shared memory of one block, dynamic and static
+
 // ---- row tiles (tile.cu)
 constexpr int kT16Zero = 8;  // zero slots after a tile, one per 16-byte bank group
 // Shared memory of a tile kernel: the slots, `hops` down hops (value and source row) and the

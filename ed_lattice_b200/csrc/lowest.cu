@@ -306,7 +306,7 @@ int launch_ritz(const TQ* Q, const double* Z, int m, int k, int64_t n, TX* X, cu
                 : K == 32 ? k_ritz_k<TQ, TX, 32>
                           : k_ritz_k<TQ, TX, 64>;
     const size_t smem = size_t(m) * K * sizeof(double);
-    if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    EDG_CHECK(allow_smem(kern, smem));
     kern<<<int(g), kLkThreads, smem, st>>>(Q, Z + size_t(r0) * m, m, nr, n, X + size_t(r0) * n);
     EDG_CUDA(cudaGetLastError());
   }

@@ -477,7 +477,7 @@ int launch(const HxvArgs<T>& a, TileArgs<T, W>& q, cudaStream_t st, int sms) {
   constexpr bool DOWN = FORM == TileForm::kDwUp || FORM == TileForm::kUpDw;
   const size_t smem = tile_smem(a.dimup, q.npal, RT * q.cap, sizeof(T) * W);
   auto kern = k_tile<T, W, FORM, LZ, PAL>;
-  if (smem > 40 * 1024) EDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  EDG_CHECK(allow_smem(kern, smem));
   // 64 registers a thread: 1024 threads per SM, in as many CTAs as the tiles leave room for
   const int per_sm = smem <= 54 * 1024 ? 4 : smem <= 111 * 1024 ? 2 : 1;
   q.nsl = int((a.dimup + 31) / 32);
