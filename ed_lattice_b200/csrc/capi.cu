@@ -229,11 +229,12 @@ int edg_sector_create(const edg_model* m, int nup, int ndw, int form, edg_sector
     return st;
   }
   // Default H x v of a real stored sector whose vectors sit in L2: the single pass (down-pass
-  // choice 3). edg_sector_autotune and edg_sector_set_kernels override it.
-  if (!s->cplx && s->form == EDG_FORM_STORED) {
-    if (s->dim <= kFusedMaxDim64) s->hxv_dw[0] = 3;
-    if (s->dim <= kFusedMaxDim32) s->hxv_dw[1] = 3;
-  }
+  // choice 3), where its kernel wins. edg_sector_autotune and edg_sector_set_kernels override it.
+  if (!s->cplx && s->form == EDG_FORM_STORED)
+    for (int f32 = 0; f32 < 2; ++f32)
+      if (single_pass_default(s->up.dim, s->dw.dim, f32 ? kFusedMaxDim32 : kFusedMaxDim64,
+                              tile_available(s, f32 ? sizeof(float) : sizeof(double), true)))
+        s->hxv_dw[f32] = 3;
   *out = s;
   return EDG_OK;
 }

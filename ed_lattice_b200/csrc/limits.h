@@ -24,6 +24,22 @@ inline size_t tile_smem(int64_t dimup, int npal, int hops, size_t elem) {
 inline bool tile_down_index(int64_t dim) { return dim < (int64_t(1) << 31); }
 
 
+// ---- default H x v of a real stored sector: the single pass or two
+// Single pass by gathers against two passes where the row tiles do not take the whole product (one
+// |value| of up hops and several of down hops, or more than 256), us, FP64:
+//   two values  3x4 (6,6), 853,776 states  61 / 41     4x4 (5,4), 7.9 M    580 / 212
+//   17 sites all-to-all (5,3), 4.2 M      975 / 350    7x2 (7,3), 364 rows  64 / 58
+//   two values  4x4 (7,2), 120 rows       120 / 168    5x3 (7,2), 105 rows  61 / 189
+//   rows beyond the tiles  17-site ring (8,2) 106 / 201, 6x3 (9,2) 649 / 859
+// So: two passes above 500,000 states, but where rows are too long for a tile, or fewer than two
+// per SM, which leaves SMs idle in either pass.
+constexpr int64_t kGatherMaxDim = 500000, kGatherMaxRows = 296;
+inline bool single_pass_default(int64_t dimup, int64_t dimdw, int64_t most, bool tiles) {
+  const int64_t dim = dimup * dimdw;
+  if (dim > most) return false;
+  return tiles || dim <= kGatherMaxDim || dimdw < kGatherMaxRows || tile_smem(dimup, 0, 0, 0) > kTileSmemMax;
+}
+
 // ---- hop tables (basis.cu)
 constexpr int kDwHops = 32;  // hops per row that the grouped down pass takes
 

@@ -143,7 +143,9 @@ int edg_hxv_d(edg_sector* s, int64_t nloc, const double* v, double* hv);
  * per H x v, *ncand their number, *best the index kept. FP64 results are the same bits for
  * every pair; the FP32 packed and Kronecker up passes change the order of a row's terms.
  * Untuned real stored sectors use the single pass (candidate 3 for FP64, 12 for FP32) up to
- * 12,000,000 (FP64) and 4,000,000 (FP32) states, other sectors candidate 0. No counterpart in the reference. */
+ * 12,000,000 (FP64) and 4,000,000 (FP32) states; above 500,000 only if it runs by row tiles (up
+ * hops of several |values|, or one |value| for each spin), DimUp exceeds a tile or DimDw < 296.
+ * Other sectors use candidate 0. No counterpart in the reference. */
 int edg_sector_autotune(edg_sector* s, int precision, int reps, double* ms, int* ncand, int* best);
 /* Pin the H x v kernel pair of this sector for one precision to candidate k of
  * edg_sector_autotune's list (0..15 for FP32, 0..3 for FP64). The tables of the non-default

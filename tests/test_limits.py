@@ -22,6 +22,9 @@ int down_index(int64_t dim) { return tile_down_index(dim); }
 int64_t groups(int64_t dim, int64_t resident, int real, int W) { return dw_group_count(dim, resident, real, W); }
 int64_t group_most(int real, int W) { return dw_group_most(real, W); }
 int64_t group_smem(int64_t rows, int real, int W) { return dw_group_smem(rows, real, W); }
+int one_pass(int64_t dimup, int64_t dimdw, int64_t most, int tiles) {
+  return single_pass_default(dimup, dimdw, most, tiles != 0);
+}
 uint64_t hops(int ns, int nel, int64_t bonds) { return hop_total(ns, nel, bonds); }
 int fits(uint64_t n) { return table_fits(n); }
 int direct(int64_t dimup, int64_t dimdw, uint64_t hu, uint64_t hd, int cplx) {
@@ -44,6 +47,7 @@ def rules(tmp_path_factory):
     r.groups.argtypes, r.groups.restype = [C.c_int64, C.c_int64, C.c_int, C.c_int], C.c_int64
     r.group_most.argtypes, r.group_most.restype = [C.c_int, C.c_int], C.c_int64
     r.group_smem.argtypes, r.group_smem.restype = [C.c_int64, C.c_int, C.c_int], C.c_int64
+    r.one_pass.argtypes = [C.c_int64, C.c_int64, C.c_int64, C.c_int]
     r.fits.argtypes = [C.c_uint64]
     r.direct.argtypes = [C.c_int64, C.c_int64, C.c_uint64, C.c_uint64, C.c_int]
     return r
@@ -118,3 +122,13 @@ def test_row_groups_fit_shared_memory(rules, real, W):
         g = rules.groups(dim, 592, real, W)
         assert 1 <= g <= dim and (g % 592 == 0 or g == dim < 592)
         assert g * most >= dim
+
+
+@pytest.mark.parametrize("case", [(924, 924, 12_000_000, 1, True), (924, 924, 12_000_000, 0, False),
+                                  (560, 560, 12_000_000, 0, True),  # 313,600 states
+                                  (4368, 1820, 12_000_000, 0, False), (4368, 1820, 4_000_000, 1, False),
+                                  (6188, 680, 12_000_000, 0, False), (11440, 120, 12_000_000, 0, True),
+                                  (24310, 136, 12_000_000, 0, True), (17550, 351, 12_000_000, 0, True),
+                                  (24310, 680, 12_000_000, 0, False)])
+def test_single_pass_is_the_default_where_its_kernel_wins(rules, case):
+    assert bool(rules.one_pass(*case[:4])) == case[4]
