@@ -263,14 +263,8 @@ struct SpinBasis {
 // at 10,306,296, 152/162 at 7,949,760, 399/386 at 19,079,424; FP32 17.4/28.8, 32.6/37.0 at
 // 2,944,656, 94/84 at 7,949,760, 247/216 at 19,079,424.
 constexpr int64_t kFusedMaxDim64 = 12000000, kFusedMaxDim32 = 4000000;
-// Complex sectors, either precision (us, one launch against two passes: complex128 326/443 at
+// Complex sectors: kFusedMaxDimC (us, one launch against two passes: complex128 326/443 at
 // 7,949,760, 342/463 at 9,018,009).
-constexpr int64_t kFusedMaxDimC = 10000000;
-// Smallest sectors, FP64 and FP32, whose single pass runs by row tiles (tile.cu): below, the
-// tiles are too few (FP32 tiles hold twice the rows) and the per-column gathers of k_hxv_fused
-// finish as soon or sooner (us, tiles against gathers: FP64 7.6/8.1 at D = 48,400, 8.5/9.8 at
-// 132,496, 10.5/15.6 at 245,025; FP32 8.7/6.7, 8.5/8.4, 9.4/12.7).
-constexpr int64_t kTileMinDim64 = 40000, kTileMinDim32 = 200000;
 constexpr int kKronThreads = 512;  // threads per CTA of the Kronecker up pass
 constexpr int kKronLL = 12;        // LL entries per low part held in registers
 // Shared memory of the Kronecker up pass: rt staged rows plus the zero slots, then the block

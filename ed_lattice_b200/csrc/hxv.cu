@@ -1601,12 +1601,17 @@ HxvArgs<T> make_args(edg_sector_s* s, const T* v, T* hv) {
   return a;
 }
 
+// Hops per state of a stored sector, both spins.
+double mean_hops(const edg_sector_s* s) {
+  return double(s->up.nnz) / double(s->up.dim) + double(s->dw.nnz) / double(s->dw.dim);
+}
+
 // Single-pass H x v (down-pass choice 3): one launch does the whole H x v; no up pass.
 // By row tiles (tile.cu) where the tile kernels apply, else the per-column gathers, which index
 // in 64 bits: edg_sector_set_kernels and edg_sector_autotune choose this pass for any size.
 template <typename T, bool LZ>
 int fused_pass(edg_sector_s* s, const HxvArgs<T>& a, cudaStream_t st, int sms) {
-  if (tile_available(s, sizeof(T), true) && s->dim >= (sizeof(T) == 8 ? kTileMinDim64 : kTileMinDim32))
+  if (tile_pays(false, sizeof(T), a.dimup, a.dimdw, mean_hops(s)) && tile_available(s, sizeof(T), true))
     return tile_real<T>(a, s->up, s->dw, TileForm::kDwUp, LZ, st, sms);
   const int64_t ntiles = a.dimdw * ((a.dimup + 31) / 32);
   const int64_t want = (ntiles + 7) / 8;
@@ -1633,10 +1638,12 @@ int hxv_apply(edg_sector_s* s, const T* v, T* hv) {
     // pass over L2-sized column slabs
     const bool stored = s->form == EDG_FORM_STORED;
     const T* vi = pick<T>(s->dw.val64i, s->dw.val32i);
-    const bool vec = reinterpret_cast<uintptr_t>(v) % (2 * sizeof(T)) == 0 && reinterpret_cast<uintptr_t>(hv) % (2 * sizeof(T)) == 0;
-    if (vec && s->dim <= kFusedMaxDimC && tile_available(s, 2 * sizeof(T), true))
+    const bool tiles = reinterpret_cast<uintptr_t>(v) % (2 * sizeof(T)) == 0 &&
+                       reinterpret_cast<uintptr_t>(hv) % (2 * sizeof(T)) == 0 &&
+                       (!stored || tile_pays(true, sizeof(T), a.dimup, a.dimdw, mean_hops(s)));
+    if (tiles && s->dim <= kFusedMaxDimC && tile_available(s, 2 * sizeof(T), true))
       return tile_cplx<T>(a, s->up, s->dw, vi, stored ? TileForm::kDwUp : TileForm::kUpDw, st, sms);
-    if (vec && s->dw.max_row <= kDwHops && s->dw.grp[0].count > 0 && tile_available(s, 2 * sizeof(T), false)) {
+    if (tiles && s->dw.max_row <= kDwHops && s->dw.grp[0].count > 0 && tile_available(s, 2 * sizeof(T), false)) {
       if (stored) {
         EDG_CHECK((dw_pass_c<T, true>(a, s->dw, vi, st)));
         return tile_cplx<T>(a, s->up, s->dw, nullptr, TileForm::kUpAdd, st, sms);

@@ -24,6 +24,35 @@ inline size_t tile_smem(int64_t dimup, int npal, int hops, size_t elem) {
 inline bool tile_down_index(int64_t dim) { return dim < (int64_t(1) << 31); }
 
 
+// Whether the tiles beat the kernels that take an element per lane and gather (k_hxv_fused,
+// k_cplx_stored); hops: mean hops per state, both spins. Stored form (the direct form's bitstring
+// kernels never win). The gathers cost a read per hop; a tile costs its staging, by many blocks
+// where rows are few, and lanes that idle where they are short (a slice has 32). us, tiles /
+// gathers, on rings (9 to 13 hops) and square lattices (14 to 24):
+//   FP64        ring 462 x 165 5.0 / 5.3, 91 x 1,001 4.4 / 4.2, 3,060 x 18 6.1 / 4.3, 15 x 5,005
+//               7.8 / 5.0;  5x3 3,003 x 15 6.4 / 7.3, 6,435 x 15 7.6 / 10.7;  4x3 220 x 220 7.6 / 8.1
+//   FP32        ring 495 x 495 6.5 / 6.6, 12,376 x 17 9.9 / 6.9;  5x3 3,003 x 105 9.7 / 14.8
+//   complex128  ring 153 x 3,060 15.9 / 14.5, 5,005 x 15 8.0 / 6.3, 18 x 18,564 21 / 10, beyond one
+//               launch 210 x 352,716 (14.8 hops) 3,520 / 2,900;  4x4 120 x 8,008 38 / 56, 4,368 x 16 7.2 / 10.4;
+//               4x3 12 x 924 4.5 / 5.9;  5x4 20 x 184,756 303 / 216
+//   complex64   ring 84 x 84 4.2 / 3.4, 120 x 560 4.7 / 3.8, 220 x 792 5.7 / 5.7, 18 x 18,564 16 / 8;
+//               4x3 924 x 66 5.9 / 6.8;  4x4 120 x 8,008 23 / 38
+// So the line lies at a number of reads, states x hops. Real sectors above 500,000 states take the
+// tiles in any shape: the two passes that ran there before lose to either (18 x 48,620 FP64 39 us
+// by tiles, 131 in two passes).
+constexpr int64_t kFusedMaxDimC = 10000000;  // complex sectors of one launch, either precision
+inline bool tile_pays(bool cplx, size_t real, int64_t dimup, int64_t dimdw, double hops) {
+  const int64_t dim = dimup * dimdw;
+  const double reads = double(dim) * hops;
+  if (!cplx && dim > 500000) return true;
+  if (dimup < 32) return cplx && real == 8 && hops >= 14.0 && dim < 32768;
+  if (!cplx && real == 8) return reads >= (dimup >= 64 && dimdw >= 64 ? 6.5e5 : 1.2e6);
+  if (!cplx) return reads >= 3.2e6;
+  if (real == 4) return reads >= 1.2e6;
+  if (dim > kFusedMaxDimC) return dimup >= 256 || hops >= 18.0;
+  return dimdw >= 32 || hops >= 10.5 || dim >= 120000;
+}
+
 // ---- default H x v of a real stored sector: the single pass or two
 // Single pass by gathers against two passes where the row tiles do not take the whole product (one
 // |value| of up hops and several of down hops, or more than 256), us, FP64:

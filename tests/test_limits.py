@@ -22,6 +22,9 @@ int down_index(int64_t dim) { return tile_down_index(dim); }
 int64_t groups(int64_t dim, int64_t resident, int real, int W) { return dw_group_count(dim, resident, real, W); }
 int64_t group_most(int real, int W) { return dw_group_most(real, W); }
 int64_t group_smem(int64_t rows, int real, int W) { return dw_group_smem(rows, real, W); }
+int pays(int cplx, int real, int64_t dimup, int64_t dimdw, double hops) {
+  return tile_pays(cplx != 0, real, dimup, dimdw, hops);
+}
 int one_pass(int64_t dimup, int64_t dimdw, int64_t most, int tiles) {
   return single_pass_default(dimup, dimdw, most, tiles != 0);
 }
@@ -48,6 +51,7 @@ def rules(tmp_path_factory):
     r.group_most.argtypes, r.group_most.restype = [C.c_int, C.c_int], C.c_int64
     r.group_smem.argtypes, r.group_smem.restype = [C.c_int64, C.c_int, C.c_int], C.c_int64
     r.one_pass.argtypes = [C.c_int64, C.c_int64, C.c_int64, C.c_int]
+    r.pays.argtypes = [C.c_int, C.c_int, C.c_int64, C.c_int64, C.c_double]
     r.fits.argtypes = [C.c_uint64]
     r.direct.argtypes = [C.c_int64, C.c_int64, C.c_uint64, C.c_uint64, C.c_int]
     return r
@@ -132,3 +136,20 @@ def test_row_groups_fit_shared_memory(rules, real, W):
                                   (24310, 680, 12_000_000, 0, False)])
 def test_single_pass_is_the_default_where_its_kernel_wins(rules, case):
     assert bool(rules.one_pass(*case[:4])) == case[4]
+
+
+# complex, bytes per real, lattice, nup, ndw; measured on both sides
+@pytest.mark.parametrize("case", [(0, 8, 15, 1, 1, 6, False), (0, 8, 18, 1, 15, 1, False), (0, 8, 9, 2, 1, 6, False),
+                                  (0, 8, 18, 1, 1, 9, True), (0, 8, 10, 1, 5, 5, True), (0, 8, 4, 4, 8, 1, True),
+                                  (0, 8, 5, 3, 7, 1, True), (0, 4, 17, 1, 11, 1, False), (0, 4, 4, 3, 4, 4, True),
+                                  (0, 4, 5, 3, 5, 2, True), (0, 4, 19, 1, 1, 12, True), (1, 8, 18, 1, 1, 6, False),
+                                  (1, 8, 5, 4, 1, 10, False), (1, 8, 15, 1, 6, 1, False), (1, 8, 4, 4, 5, 1, True),
+                                  (1, 8, 8, 1, 4, 4, True), (1, 8, 21, 1, 2, 10, False), (1, 8, 19, 1, 3, 9, True),
+                                  (1, 4, 9, 1, 3, 3, False), (1, 4, 4, 3, 6, 2, True), (1, 4, 17, 1, 1, 7, False),
+                                  (1, 4, 21, 1, 2, 10, True)])
+def test_tiles_run_where_they_win(rules, case):
+    cplx, real, lx, ly, nup, ndw, want = case
+    ns, nb = lx * ly, _bonds(E.square_lattice(lx, ly))
+    up, dw = math.comb(ns, nup), math.comb(ns, ndw)
+    hops = rules.hops(ns, nup, nb) / up + rules.hops(ns, ndw, nb) / dw
+    assert bool(rules.pays(cplx, real, up, dw, hops)) == want
