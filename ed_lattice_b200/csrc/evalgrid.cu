@@ -9,6 +9,11 @@
 // Bound by FP64 arithmetic, most of it in the division, so eight poles share one: with the
 // products of pairs, fours and all eight denominators, each reciprocal is a product of the
 // others and of 1/all (2.6 products and an eighth of a division per term instead of a division).
+// Such a reciprocal carries a few roundings more, the sums fewer: groups are summed apart, chunks
+// by pairs. rms error in 1e-16 of the sum of magnitudes, against 64-bit mantissas, with a division
+// per term and 64 chunks one after the other / now: 8 poles 0.83 / 0.77, 16 0.92 / 0.89, 64
+// 1.41 / 0.69, 150 1.21 / 0.64, 1,200 1.25 / 0.49, 120,000 1.48 / 0.46. Up to 64 poles, where the
+// rounding of the quotients counts, each term has its own division (8 poles 1.15 without).
 // 120,000 poles x 9,096 frequencies: a division per term 1176 us, per four terms 852, per eight
 // 740 with the range tested per group, 662 with it tested per tile of poles.
 #include <algorithm>
@@ -21,6 +26,7 @@ namespace {
 constexpr int kEvalThreads = 256;
 constexpr int kEvalChunks = 128;  // most pole chunks (second grid dimension)
 constexpr int kEvalTile = 1024;   // poles staged in shared memory at a time
+constexpr int kEvalOwn = 64;      // most poles whose terms have a division each
 
 __device__ __forceinline__ void add_term(double w, double d, double a, double y, double& re, double& im) {
   const double s = w / a;
@@ -80,7 +86,7 @@ __global__ void __launch_bounds__(kEvalThreads) k_eval_poles(const double* __res
     // y^2 <= a <= (|x| + max |p|)^2 + y^2 for every pole of the tile
     const double far = fabs(x) + pm;
     int q = 0;
-    if (yy >= 1e-35 && far * far + yy <= 1e35)
+    if (npoles > kEvalOwn && yy >= 1e-35 && far * far + yy <= 1e35)
       for (; q + 8 <= cnt; q += 8) add_eight(sp + q, sw + q, x, y, yy, re, im);
     for (; q < cnt; ++q) {
       const double d = x - sp[q];
@@ -96,13 +102,25 @@ __global__ void __launch_bounds__(kEvalThreads) k_eval_poles(const double* __res
 __global__ void k_eval_sum(const double* __restrict__ part, int nchunks, int64_t nz, double* __restrict__ out) {
   const int64_t m = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (m >= nz) return;
-  double re = 0.0, im = 0.0;
-  for (int c = 0; c < nchunks; ++c) {
-    re += part[(int64_t(c) * nz + m) * 2];
-    im += part[(int64_t(c) * nz + m) * 2 + 1];
-  }
-  out[2 * m] = re;
-  out[2 * m + 1] = im;
+  double re[8], im[8];  // every eighth chunk, then by pairs
+#pragma unroll
+  for (int i = 0; i < 8; ++i) re[i] = im[i] = 0.0;
+  for (int c = 0; c < nchunks; c += 8)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (c + i < nchunks) {
+        re[i] += part[(int64_t(c + i) * nz + m) * 2];
+        im[i] += part[(int64_t(c + i) * nz + m) * 2 + 1];
+      }
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      re[i] += re[i + h];
+      im[i] += im[i + h];
+    }
+  out[2 * m] = re[0];
+  out[2 * m + 1] = im[0];
 }
 
 }  // namespace
