@@ -259,9 +259,10 @@ struct SpinBasis {
 
 // Largest sector that defaults to the single-pass H x v, FP64 and FP32: its source rows must
 // come from L2, and the two-pass kernels' down pass, which sweeps L2-sized column slabs, wins
-// beyond. Measured (us, single pass against two passes): FP64 24.6/43.2 at D = 853,776, 183/215
-// at 10,306,296, 152/162 at 7,949,760, 399/386 at 19,079,424; FP32 17.4/28.8, 32.6/37.0 at
-// 2,944,656, 94/84 at 7,949,760, 247/216 at 19,079,424.
+// beyond. Measured (us, single pass / two passes, both by tiles): FP64 21.9/30.7 on 3x4 (6,6),
+// 853,776 states, 146/152 on 4x4 (4,5), 7.9 M, 174/215 on 7x2 (6,7), 10.3 M, 201/203 on (7,7),
+// 11.8 M, 405/362 on 4x4 (5,5), 19.1 M; FP32 17.7/26.3, 13-site ring (6,6), 2.9 M, 33.6/34.0,
+// 4x4 (4,5) 94/76, (5,5) 245/188.
 constexpr int64_t kFusedMaxDim64 = 12000000, kFusedMaxDim32 = 4000000;
 // Complex sectors: kFusedMaxDimC (us, one launch against two passes: complex128 326/443 at
 // 7,949,760, 342/463 at 9,018,009).
@@ -326,10 +327,11 @@ struct edg_sector_s {
   int last_n32 = 0, last_n64 = 0;  // H x v applications of the last ground-state run per precision
   // H x v kernel choice per vector precision ([0] FP64, [1] FP32), set by edg_sector_autotune:
   // down pass 0 = hop-balanced row groups, 1 = block-staged (one CTA per SM), 2 = block-staged
-  // (two CTAs per SM), 3 = single pass (k_hxv_fused: the whole H x v, no up pass); up pass
-  // (FP32) 0 = 32-bit SELL schedule, 1 = packed 16-bit schedule with negated copies, 2 = packed
-  // 16-bit schedule with sign bits, 3 = Kronecker schedule. Until tuned: 3/0 for real stored
-  // sectors of at most kFusedMaxDim64 / kFusedMaxDim32 states, else 0/0.
+  // (two CTAs per SM), 3 = single pass, no up pass (k_tile kDwUp, or k_hxv_fused where the tiles do
+  // not apply or do not pay); up pass (FP32) 0 = row tiles (k_tile kUpAdd; k_up_smem and k_up_split
+  // for rows and tables that those do not take), 1 = packed 16-bit schedule with negated copies,
+  // 2 = packed 16-bit schedule with sign bits, 3 = Kronecker schedule. Until tuned: 3/0 for real
+  // stored sectors where single_pass_default says so, else 0/0.
   int hxv_dw[2] = {0, 0};
   int hxv_up[2] = {0, 0};
 };
@@ -437,7 +439,7 @@ int lanczos_step_b2_cols(cudaStream_t st, int ncols, const int* active, T* w, co
 template <typename T>
 int scale_into_cols(cudaStream_t st, int ncols, const int* active, T* dst, const T* src, int64_t vstride,
                     const double* b, int64_t sstride, int64_t n);
-// *out = |x| (FP64, fixed reduction grid; partial holds kRedBlocks values)
+// *out = |x| (FP64, fixed reduction grid; partial: a reduction scratch of kRedSlots doubles)
 int norm_dev(cudaStream_t st, const double* x, int64_t n, double* partial, double* out);
 // dst = TD(src * scale); dst and src must not overlap (scale_inplace_dev scales in place)
 template <typename TD, typename TS>

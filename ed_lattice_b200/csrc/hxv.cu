@@ -763,7 +763,8 @@ __global__ void __launch_bounds__(256) k_hxv_fused(HxvArgs<T> a, int64_t ntiles)
 }
 
 // Down-spin pass, balanced persistent form. CTA g owns the rows of group g (rows grouped on
-// the host so every group carries the same total number of hops); their hop lists sit in
+// the host so every group carries the same total number of hops, one group per resident CTA or,
+// where rows are very many, for each of several turns); their hop lists sit in
 // shared memory. All CTAs sweep the column slabs (32*VEC columns) in the same order; inside
 // a CTA the warps take the group's rows from a shared counter, and a CTA barrier closes
 // each slab. Equal work per CTA keeps the whole grid within a few slabs of each other, so
@@ -1069,7 +1070,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_dw_blk(HxvArgs<T> a, const ui
 }
 
 // ---------------------------------------------------------------- direct (on-the-fly) form
-// For the sectors that the row tiles do not take. No tables: each thread derives its hops from the bitstrings, as directMatVec does, with
+// For the sectors that the row tiles do not take (direct_tables). No tables: each thread derives its hops from the bitstrings, as directMatVec does, with
 // ranks from the combinatorial number system instead of binary_search. Bonds arrive
 // sorted by 2^b - 2^a so that sources come out in ascending rank.
 struct DirectArgsHdr {
@@ -1673,8 +1674,9 @@ int hxv_apply(edg_sector_s* s, const T* v, T* hv) {
     EDG_CHECK((dw_pass<T, true, false>(a, s->dw, st, sms)));
     EDG_CHECK((up_pass<T, false, false>(a, s, st, sms, nullptr)));
   } else {
-    // By row tiles (4x4 (6,6), FP64 / FP32: 1.44 / 0.61 ms, against 6.44 / 5.62 by k_direct_rows,
-    // whose up gathers scatter over global memory; 3x4 (6,6) 25 / 19 us against 126 / 119). The bitstring kernels serve the rows and hop lists that those do not take.
+    // By row tiles (4x4 (6,6), FP64 / FP32: 1.16 / 0.60 ms, against 6.44 / 5.62 by k_direct_rows,
+    // whose up gathers scatter over global memory; 3x4 (6,6) 22.5 / 18.5 us against 126 / 119). The
+    // bitstring kernels serve the sectors that keep no tables (direct_tables) and longer hop lists.
     if (s->dim <= (sizeof(T) == 8 ? kFusedMaxDim64 : kFusedMaxDim32) && tile_available(s, sizeof(T), true))
       return tile_real<T>(a, s->up, s->dw, TileForm::kUpDw, false, st, sms);
     if (s->dw.max_row <= kDwHops && s->dw.grp[0].count > 0 && tile_available(s, sizeof(T), false)) {

@@ -444,8 +444,10 @@ int gs_run(edg_sector_s* s, const double* dv0, int maxit, double tol, std::vecto
     // While the last test was far from convergence (its error estimate more than 100x the
     // target 0.1 tol |E0|), step j+1 is queued before the host waits for step j, so the GPU
     // goes from step to step; near convergence the test comes first, so no step is wasted.
-    // Per call, U = 8, FP64, the wait first and a QL iteration every step -> this: 245,025
-    // states 20.7 -> 7.9 ms, 853,776 18.4 -> 8.5, 9.0 M 53.9 -> 40.3, 64 M 249 -> 245.
+    // Per call, U = 8, the wait first and a QL iteration every step -> this, over three disordered
+    // lattices (110 to 140 products, repeats within 2 %): FP64 245,025 states 17.1-25.1 -> 7.0-9.1
+    // ms, 853,776 21.1-24.8 -> 9.3-10.8, 9.0 M 41.6-51.5 -> 38.4-45.2; FP32 with refinement 64 M
+    // (169 to 279 products) 195-352 -> 193-350.
     queued = j + 1 < maxit && err_prev > 10.0 * tol * std::fabs(eold);
     if (queued) {
       EDG_CHECK(R.advance_dev(j));

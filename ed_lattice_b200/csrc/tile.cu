@@ -25,8 +25,8 @@
 // Measured, before (32-bit SELL entries, two FP32 or two FP64 rows) and now, us:
 //   up pass, 4x4 (8,8)  FP32  1025 -> 808     4x4 (7,7) FP64  1862 -> 1294
 //   up pass, 5x3 (7,8)  FP64   570 -> 397     fused Lanczos 4x4 (6,6) FP64  1084 -> 804
-//   whole product, 3x4 (6,6) FP64: two passes 44.0 -> 22.3; 12 Lanczos columns 491 -> 187
-//   complex128 4x4 (5,5): 2433 (one thread per element, L1 gathers) -> 1157 in two passes;
+//   whole product, 3x4 (6,6) FP64: two passes 44.0 -> 21.9; 12 Lanczos columns 491 -> 187
+//   complex128 4x4 (5,5): 2433 (one thread per element, L1 gathers) -> 923 in two passes;
 //   3x4 (6,6) 81 -> 44, 4x4 (4,5) 825 -> 326 in one launch
 #include <algorithm>
 #include <type_traits>
@@ -123,7 +123,7 @@ __device__ __forceinline__ void elem_fma(const T* h, const T* x, T* acc) {
 
 // A down hop of a row: the value and the first element of the source row. The plain product over
 // tables of one |value| keeps the element with the value's sign in bit 31 instead (PACK): four
-// hops per shared-memory load (3x4 (6,6) FP64 22.3 -> 20.4 us). The Lanczos-fused one, short of
+// hops per shared-memory load (8 % of the product on 3x4 (6,6), FP64). The Lanczos-fused one, short of
 // registers, is slower with it (12 columns of 731,808: 202 -> 217 us).
 template <typename T, int W>
 struct alignas(8) Hop {

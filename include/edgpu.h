@@ -135,7 +135,7 @@ int edg_hxv_d(edg_sector* s, int64_t nloc, const double* v, double* hv);
  * (nup = 4 for FP32, 1 for FP64): down 0 hop-balanced row groups, 1 block-staged rows (one
  * CTA per SM), 2 block-staged rows (two CTAs per SM), 3 the single-pass H x v (the whole
  * product in one launch, for vectors that sit in L2; the up choice is then unused); up (FP32)
- * 0 row tiles of 16-byte slots over a 16-bit schedule (rows of up to about 14,400 columns;
+ * 0 row tiles of 16-byte slots over a 16-bit schedule (rows of up to 14,343 columns;
  * 32-bit SELL schedule beyond),
  * 1 packed 16-bit schedule with negated copies, 2 packed 16-bit schedule with sign bits,
  * 3 Kronecker schedule (hops inside the low or the high half of the sites from per-half
